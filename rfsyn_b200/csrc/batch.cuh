@@ -208,6 +208,8 @@ static inline int qb_prepare() {
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+constexpr int V_BATCH_NT = 192;  // threads of the vector sweep's CTAs
+
 struct rfb_batch {
     std::vector<rfb_engine *> m;  // members (owned)
     int prec = RFB_FP32;
@@ -223,6 +225,11 @@ struct rfb_batch {
     BatchItem *d_items[3] = {};    // interior, x slab, edge (uni: every item in the edge list)
     int n_items[3] = {};
     int uni = 0;
+    // mode 5: the vector sweep's items of every scene, shapes and maps
+    VItem *d_vitems = nullptr;
+    int n_vitems = 0, n_vplain = 0, v_nt = 0, v_smem = 0;
+    VShape *d_vshapes = nullptr;
+    VMaps *d_vmaps[2] = {};
     int2 *d_lblocks = nullptr;
     int n_lblocks = 0;
     void *d_probes = nullptr;
@@ -245,9 +252,112 @@ static void batch_free_plan(rfb_batch *b) {
         b->g1[q] = b->gk[q] = nullptr;
         dfree(b->d_maps[q]);
         b->d_maps[q] = nullptr;
+        dfree(b->d_vmaps[q]);
+        b->d_vmaps[q] = nullptr;
     }
     dfree(b->d_dims);
     b->d_dims = nullptr;
+    dfree(b->d_vitems);
+    dfree(b->d_vshapes);
+    b->d_vitems = nullptr;
+    b->d_vshapes = nullptr;
+    b->n_vitems = b->n_vplain = 0;
+}
+
+// Plan of mode 5, the vector sweep of every scene in one launch: per scene
+// the tile of at most `threads` threads that spends the fewest threads on the
+// grid, and one segment length for the batch by the rule of v_rule.  Items
+// of one kind together, the costly kinds first.
+static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
+    batch_free_plan(b);
+    const size_t n = b->m.size();
+    std::vector<VShape> shapes(n);
+    std::vector<VMaps> maps[2];
+    std::vector<VItem> items;
+    maps[0].resize(n);
+    maps[1].resize(n);
+    double planes = 0;
+    int smem = 0;
+    for (size_t s = 0; s < n; s++) {
+        rfb_engine *e = b->m[s];
+        if (e->g.periodic & 6u) {
+            rfb_set_error("batch scene %zu: a tile halo wraps around a periodic y or z axis", s);
+            return -1;
+        }
+        if (!v_fits(e)) {
+            rfb_set_error("batch scene %zu too large for the vector sweep (32-bit offsets)", s);
+            return -1;
+        }
+        const int N = e->prec == RFB_FP64 ? 2 : 4;
+        int cj, ck, ci;
+        v_extents(e, e->active, &cj, &ck, &ci);
+        const int nvk = (ck + N - 1) / N;
+        long long best = -1, best_tiles = 0;
+        for (int nk = 1, pv = 0; nk <= nvk; nk++) {
+            const int nv = (nvk + nk - 1) / nk;
+            if (nv == pv) continue;
+            pv = nv;
+            for (int tr = std::min(cj, threads / (nv + 1) - 1); tr >= 1; tr--) {
+                const int nj = (cj + tr - 1) / tr;
+                if (tr > 1 && nj == (cj + tr - 2) / (tr - 1)) continue;
+                VShape t;
+                if (!v_layout(e, t, nv, tr, cj, ck, threads)) continue;
+                const long long tiles = (long long)((nvk + nv - 1) / nv) * nj;
+                const long long cost = tiles * ((tr + 1) * (nv + 1) + threads);
+                if (best < 0 || cost < best) {
+                    best = cost;
+                    best_tiles = tiles;
+                    shapes[s] = t;
+                }
+            }
+        }
+        if (best < 0) {
+            rfb_set_error("batch scene %zu: no tile fits", s);
+            return -1;
+        }
+        planes += (double)best_tiles * ci;
+        smem = std::max(smem, shapes[s].smem);
+        if (v_encode(e, shapes[s]) != 0) return -1;
+        maps[0][s] = e->vmaps[0];
+        maps[1][s] = e->vmaps[1];
+    }
+    smem = (int)round_up(smem, 16);
+    const double slots = 148.0 * v_slots(threads, smem + (b->prec == RFB_FP64 ? v_args_bytes<double>() : v_args_bytes<float>()));
+    if (seg <= 0) {
+        const double per_slot = planes / slots;
+        seg = std::max(1, (int)ceil(per_slot <= 16 ? per_slot : per_slot / std::max(2.0, ceil(per_slot / 32))));
+    }
+    b->n_vplain = 0;
+    for (size_t s = 0; s < n; s++) {
+        int cj, ck, ci;
+        v_extents(b->m[s], b->m[s]->active, &cj, &ck, &ci);
+        const int sg = std::min(seg, v_max_seg(b->m[s]));
+        v_items(b->m[s], shapes[s], ci, sg, sg, (int)s, items, &b->n_vplain);
+    }
+    auto rank = [](const VItem &x) { return x.kind & V_X ? 0 : 4 - x.kind; };
+    std::stable_sort(items.begin(), items.end(), [&](const VItem &x, const VItem &y) {
+        if (rank(x) != rank(y)) return rank(x) < rank(y);
+        return x.ie - x.ib > y.ie - y.ib;
+    });
+    b->mode = 5;
+    b->uni = 1;
+    b->tj = threads;
+    b->ns = V_NH;
+    b->seg_int = b->seg_edge = seg;
+    b->v_nt = threads;
+    b->v_smem = smem;
+    b->n_vitems = (int)items.size();
+    CK(dmalloc(&b->d_vitems, items.size() * sizeof(VItem)));
+    CK(cudaMemcpy(b->d_vitems, items.data(), items.size() * sizeof(VItem), cudaMemcpyHostToDevice));
+    CK(dmalloc(&b->d_vshapes, n * sizeof(VShape)));
+    CK(cudaMemcpy(b->d_vshapes, shapes.data(), n * sizeof(VShape), cudaMemcpyHostToDevice));
+    for (int q = 0; q < 2; q++) {
+        CK(dmalloc(&b->d_vmaps[q], n * sizeof(VMaps)));
+        CK(cudaMemcpy(b->d_vmaps[q], maps[q].data(), n * sizeof(VMaps), cudaMemcpyHostToDevice));
+    }
+    return 0;
+fail:
+    return -1;
 }
 
 // Work lists and per-scene tensor maps / dims of one plan.
@@ -323,6 +433,11 @@ fail:
 template <typename T>
 static void batch_sweep(rfb_batch *b, int par) {
     const Args<T> *args = (const Args<T> *)b->d_args[par];
+    if (b->mode == 5) {
+        v_launch_b<T>(args, b->d_vshapes, b->d_vmaps[par], b->d_vitems, b->n_vitems, b->v_nt, b->v_smem, b->d_err,
+                      b->stream);
+        return;
+    }
     const TmaMaps *maps = b->d_maps[par];
     if (b->uni) {
         launch_qb<5, T>(args, b->d_dims, maps, b->tj, b->ns, b->d_items[2], b->n_items[2], b->d_queue + 2, b->d_err,
@@ -350,7 +465,8 @@ static void batch_rest(rfb_batch *b, int par) {
 }
 
 static int batch_launches_per_step(const rfb_batch *b) {
-    return (b->n_items[0] > 0) + (b->n_items[1] > 0) + (b->n_items[2] > 0) + (b->n_lblocks > 0) + 1;
+    const int sweep = b->mode == 5 ? 1 : (b->n_items[0] > 0) + (b->n_items[1] > 0) + (b->n_items[2] > 0);
+    return sweep + (b->n_lblocks > 0) + 1;
 }
 
 static void batch_enqueue_step(rfb_batch *b, int par) {
@@ -391,116 +507,21 @@ fail:
     return -1;
 }
 
-// Picks the plan (tile height, ring depth, tile origins, segment lengths) by
-// timing a few batched sweeps of each candidate; every candidate computes
-// bit-identical fields, so the choice changes speed only.
-// Plans chosen for batches of the same scene geometries (in order), so that
-// a batch built again -- the next set of examples of a stage, an end-to-end
-// run -- skips the tuning.
-struct BatchCand {
-    int tj, ns, mode, si, se, uni;
-};
-static std::mutex g_btune_mu;
-static std::vector<std::pair<std::vector<long long>, BatchCand>> g_btune_cache;
-
-static std::vector<long long> batch_key(const rfb_batch *b) {
-    std::vector<long long> key = {b->prec, (long long)b->m.size()};
-    for (const rfb_engine *e : b->m) {
-        const rfb_geom_t &g = e->g;
-        key.insert(key.end(), {g.nx, g.ny, g.nz, (long long)g.periodic, e->active, e->cpml.on});
-        if (e->cpml.on)
-            for (int a = 0; a < 3; a++)
-                key.insert(key.end(), {e->cpml.eh[a].lo, e->cpml.eh[a].hi, e->cpml.em[a].lo, e->cpml.em[a].hi});
-        key.push_back(e->scene.n_skip);
-        for (int s = 0; s < e->scene.n_skip; s++) key.push_back(e->scene.skip[s]);
-    }
-    return key;
-}
-
-static int batch_autotune(rfb_batch *b) {
-    using Cand = BatchCand;
-    std::vector<Cand> cands;
-    const InteriorVariant *v = b->prec == RFB_FP32 ? kQVariantsFp32 : kQVariantsFp64;
-    const size_t nv = b->prec == RFB_FP32 ? std::size(kQVariantsFp32) : std::size(kQVariantsFp64);
-    bool wrap_yz = false;
-    for (const rfb_engine *e : b->m) wrap_yz |= (e->g.periodic & 6u) != 0;
-    // two stages: variant, tile origins and queue form at (64, 32)-plane
-    // items, then the segment lengths of the winner
-    for (size_t q = 0; q < nv; q++)
-        for (int mode = 2; mode <= (wrap_yz ? 3 : 4); mode++)
-            for (int uni : {0, 1}) cands.push_back(Cand{v[q].tj, v[q].ns, mode, 64, 32, uni});
+// The plan: mode 5 by rule, or the one RFSYN_FDTD_PLAN names -- a work-queue
+// sweep, or "threads,stages,seg_interior,seg_edge,5".  Every plan computes
+// bit-identical fields.
+static int batch_plan(rfb_batch *b) {
     const char *ov = rfb_plan_override();
-    if (ov) {
-        int a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0;
-        const int nov = sscanf(ov, "%d,%d,%d,%d,%d,%d", &a1, &a2, &a3, &a4, &a5, &a6);
-        if (nov < 5 || a5 < 2 || a3 <= 0 || a4 <= 0 || a6 < 0 || a6 > 1 || !plan_variant_known(b->prec, a1, a2, a5)) {
-            rfb_set_error("sweep plan \"%s\" names no work-queue sweep variant", ov);
-            return -1;
-        }
-        return batch_build_plan(b, a1, a2, a5, a3, a4, a6);
+    if (!ov) return batch_build_vplan(b, V_BATCH_NT, 0);
+    int a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0;
+    const int nov = sscanf(ov, "%d,%d,%d,%d,%d,%d", &a1, &a2, &a3, &a4, &a5, &a6);
+    if (nov >= 5 && a5 == 5 && a3 > 0 && a1 >= 32 && a1 <= V_NT && a1 % 32 == 0) return batch_build_vplan(b, a1, a3);
+    if (nov < 5 || a5 < 2 || a5 > 4 || a3 <= 0 || a4 <= 0 || a6 < 0 || a6 > 1 ||
+        !plan_variant_known(b->prec, a1, a2, a5)) {
+        rfb_set_error("sweep plan \"%s\" names no work-queue or vector sweep variant", ov);
+        return -1;
     }
-    const std::vector<long long> key = batch_key(b);
-    {
-        std::lock_guard<std::mutex> lock(g_btune_mu);
-        for (const auto &kv : g_btune_cache)
-            if (kv.first == key) {
-                const Cand &c = kv.second;
-                return batch_build_plan(b, c.tj, c.ns, c.mode, c.si, c.se, c.uni);
-            }
-    }
-    Cand best = cands[0];
-    const size_t first_stage = cands.size();
-    float best_ms = 1e30f;
-    cudaEvent_t t0 = nullptr, t1 = nullptr;
-    int par = 0;
-    CK(cudaEventCreate(&t0));
-    CK(cudaEventCreate(&t1));
-    for (size_t ci = 0; ci < cands.size(); ci++) {
-        const Cand c = cands[ci];
-        if (batch_build_plan(b, c.tj, c.ns, c.mode, c.si, c.se, c.uni) != 0) goto fail;
-        for (int w = 0; w < 5; w++) {
-            if (w == 2) CK(cudaEventRecord(t0, b->stream));
-            if (b->prec == RFB_FP64) batch_sweep<double>(b, par);
-            else batch_sweep<float>(b, par);
-            par ^= 1;
-        }
-        CK(cudaEventRecord(t1, b->stream));
-        CK(cudaEventSynchronize(t1));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, t0, t1));
-        if (ms < best_ms) {
-            best_ms = ms;
-            best = c;
-        }
-        if (ci + 1 == first_stage)
-            for (int si : {32, 64})
-                for (int se : {16, 32})
-                    if (si != best.si || se != best.se)
-                        cands.push_back(Cand{best.tj, best.ns, best.mode, si, se, best.uni});
-    }
-    cudaEventDestroy(t0);
-    cudaEventDestroy(t1);
-    {
-        int err = 0;
-        CK(cudaMemcpy(&err, b->d_err, sizeof err, cudaMemcpyDeviceToHost));
-        if (err) {
-            rfb_set_error("batch: %s", sweep_error_text(err));
-            return -1;
-        }
-    }
-    {
-        std::lock_guard<std::mutex> lock(g_btune_mu);
-        g_btune_cache.push_back({key, best});
-    }
-    if (batch_build_plan(b, best.tj, best.ns, best.mode, best.si, best.se, best.uni) != 0) return -1;
-    // the tuning sweeps advanced the fields: start from the zero state again
-    if (rfb_batch_reset(b) != 0) return -1;
-    CK(cudaStreamSynchronize(b->stream));
-    return 0;
-fail:
-    if (t0) cudaEventDestroy(t0);
-    if (t1) cudaEventDestroy(t1);
-    return -1;
+    return batch_build_plan(b, a1, a2, a5, a3, a4, a6);
 }
 
 extern "C" void rfb_batch_destroy(rfb_batch_t *b) {
@@ -629,9 +650,9 @@ extern "C" rfb_batch_t *rfb_batch_create(rfb_engine_t **members, size_t n, void 
     if ((b->prec == RFB_FP64 ? batch_upload_args<double>(b) : batch_upload_args<float>(b)) != 0) goto fail;
     CK(cudaDeviceSynchronize());
     {
-        const double t_tune = rfb_now();
-        const int rc = batch_autotune(b);
-        rfb_trace("batch: plan (tuned or cached)", t_tune);
+        const double t_plan = rfb_now();
+        const int rc = batch_plan(b);
+        rfb_trace("batch: plan", t_plan);
         if (rc != 0) goto fail;
     }
     return b;
@@ -774,9 +795,9 @@ extern "C" int rfb_batch_info(rfb_batch_t *b, rfb_batch_info_t *out) {
     out->unified = b->uni;
     out->seg_interior = b->seg_int;
     out->seg_edge = b->seg_edge;
-    out->items_interior = b->n_items[0];
+    out->items_interior = b->mode == 5 ? b->n_vplain : b->n_items[0];
     out->items_xslab = b->n_items[1];
-    out->items_edge = b->n_items[2];
+    out->items_edge = b->mode == 5 ? b->n_vitems - b->n_vplain : b->n_items[2];
     out->launches_per_step = batch_launches_per_step(b);
     return 0;
 }

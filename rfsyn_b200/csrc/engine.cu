@@ -18,6 +18,7 @@
 #include "fused.cuh"
 #include "tma.cuh"
 #include "sweep.cuh"
+#include "vsweep.cuh"
 #include "energy.cuh"
 #include "iq.cuh"
 #include "sphere_frac.cuh"
@@ -253,8 +254,12 @@ static long long pitch_for(int nz, size_t esz) {
 // ---------------------------------------------------------------------------
 // CPML on the device: profiles in the run precision, psi over slabs only.
 // ---------------------------------------------------------------------------
+// Slab cells [0, lo) and [hi, len) of an axis (ns of them), and where a psi
+// array keeps them: `slots` slots along its slab axis, low cells at slot q,
+// high cells at slot q + off.
 struct SlabExt {
     int lo, hi, ns;
+    int slots, off;
 };
 
 // Leading / trailing non-identity runs of a profile (kappa_inv, b, a) =
@@ -275,7 +280,20 @@ static SlabExt slab_extent(const double *kinv, const double *b, const double *a,
         s.lo = lead; s.hi = len - trail;
     }
     s.ns = s.lo + (len - s.hi);
+    s.slots = s.ns;
+    s.off = s.lo - s.hi;
     return s;
+}
+
+// z slabs: the slots of a psi row start on vectors of v cells as the cells of
+// a field row do, so that a vector of cells finds its psi in one aligned
+// vector; slots beside the slab cells hold zero.  Where the two slabs share
+// a vector (a grid little longer than its CPML) every cell keeps its own
+// position.
+static void align_slots(SlabExt &s, int len, int v) {
+    const int lo_up = (s.lo + v - 1) / v * v, hi_dn = s.hi / v * v, len_up = (len + v - 1) / v * v;
+    s.off = lo_up > hi_dn ? 0 : lo_up - hi_dn;
+    s.slots = s.hi < len ? len_up + s.off : lo_up;
 }
 
 struct DevCpml {
@@ -330,21 +348,28 @@ static int devcpml_init(DevCpml &c, const rfb_geom_t *g, const rfb_cpml_desc_t *
         }
     {
         std::vector<unsigned char> stage(prof_bytes, 0);
+        const size_t v = 16 / esz;
         for (int a = 0; a < 3; a++) {
             const double *src[6] = {d->kinv_m[a], d->b_m[a], d->a_m[a], d->kinv_h[a], d->b_h[a], d->a_h[a]};
             for (int q = 0; q < 6; q++) {
                 const size_t len = q < 3 ? (size_t)n[a] + 1 : (size_t)n[a];
                 unsigned char *dst = stage.data() + prof_off[a][q];
+                // whole vectors: the identity (1, 1, 0) beyond the profile's end
+                const double pad = q % 3 == 2 ? 0.0 : 1.0;
                 if (prec == RFB_FP64) {
                     memcpy(dst, src[q], len * 8);
+                    for (size_t k = len; k % v; k++) reinterpret_cast<double *>(dst)[k] = pad;
                 } else {
                     float *f = reinterpret_cast<float *>(dst);
                     for (size_t k = 0; k < len; k++) f[k] = (float)src[q][k];
+                    for (size_t k = len; k % v; k++) f[k] = (float)pad;
                 }
             }
             c.em[a] = slab_extent(d->kinv_m[a], d->b_m[a], d->a_m[a], n[a] + 1);
             c.eh[a] = slab_extent(d->kinv_h[a], d->b_h[a], d->a_h[a], n[a]);
         }
+        align_slots(c.em[2], n[2] + 1, (int)(16 / esz));
+        align_slots(c.eh[2], n[2], (int)(16 / esz));
         if (dmalloc(&c.prof_base, prof_bytes) != cudaSuccess ||
             cudaMemcpy(c.prof_base, stage.data(), prof_bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
             rfb_set_error("cpml profile upload failed");
@@ -353,7 +378,7 @@ static int devcpml_init(DevCpml &c, const rfb_geom_t *g, const rfb_cpml_desc_t *
         for (int a = 0; a < 3; a++)
             for (int q = 0; q < 6; q++) c.prof[a][q] = static_cast<char *>(c.prof_base) + prof_off[a][q];
     }
-    // extents of a psi array with slab axis ax and ns slab cells
+    // extents of a psi array with slab axis ax and ns slots along it
     auto bytes = [&](int ax, int ns) -> size_t {
         size_t e;
         if (ax == 0) e = (size_t)ns * (g->ny + 1) * pitch;
@@ -365,8 +390,8 @@ static int devcpml_init(DevCpml &c, const rfb_geom_t *g, const rfb_cpml_desc_t *
     size_t off_e[6], off_h[2][6], total = 0;
     for (int p = 0; p < 6; p++) {
         const int ax = psi_axis_e(p), ah = psi_axis_h(p);
-        c.psi_e_bytes[p] = bytes(ax, c.em[ax].ns);
-        c.psi_h_bytes[p] = bytes(ah, c.eh[ah].ns);
+        c.psi_e_bytes[p] = bytes(ax, c.em[ax].slots);
+        c.psi_h_bytes[p] = bytes(ah, c.eh[ah].slots);
         off_e[p] = total;
         total += align256(c.psi_e_bytes[p]);
         for (int b = 0; b < nbuf_h; b++) {
@@ -401,8 +426,10 @@ static void fill_cpml_args(Args<T> &a, const DevCpml &c, int hin, int hout) {
         a.kinv_h[ax] = (const T *)c.prof[ax][3];
         a.b_h[ax] = (const T *)c.prof[ax][4];
         a.a_h[ax] = (const T *)c.prof[ax][5];
-        a.lo_m[ax] = c.em[ax].lo; a.hi_m[ax] = c.em[ax].hi; a.ns_m[ax] = c.em[ax].ns;
-        a.lo_h[ax] = c.eh[ax].lo; a.hi_h[ax] = c.eh[ax].hi; a.ns_h[ax] = c.eh[ax].ns;
+        a.lo_m[ax] = c.em[ax].lo; a.hi_m[ax] = c.em[ax].hi; a.ns_m[ax] = c.em[ax].slots;
+        a.off_m[ax] = c.em[ax].off;
+        a.lo_h[ax] = c.eh[ax].lo; a.hi_h[ax] = c.eh[ax].hi; a.ns_h[ax] = c.eh[ax].slots;
+        a.off_h[ax] = c.eh[ax].off;
     }
     for (int p = 0; p < 6; p++) {
         a.psi_e[p] = (T *)c.psi_e[p];
@@ -645,6 +672,7 @@ struct rfb_engine {
     int launches_per_step = 0;
     FusedPlan plan;
     TmaMaps tmaps[2];       // tensor maps of the input buffers per parity (TMA interior sweep)
+    VMaps vmaps[2];         // and of the vector sweep (mode 5)
     int *d_err = nullptr;   // set by a sweep whose copies did not complete in time
     double *d_energy = nullptr;  // energy audit: block partials + result
     float *d_iq = nullptr;       // stage output: n_steps I/Q pairs, then the noise scale (a double)
@@ -807,12 +835,18 @@ static void launch_rest(rfb_engine *e, const Args<T> &a, int par, cudaStream_t s
     if (!edge_on_third_stream(e)) launch_edge<T>(a, e->plan, st);
 }
 
-// One fused sweep: the interior kinds on the engine stream, the slab /
+// One fused sweep.  Mode 5: one launch of the vector sweep.  Other modes: the
+// interior kinds on the engine stream, the slab /
 // boundary kinds on the second stream, side by side (they touch disjoint
 // cells); a work-queue plan's cp.async-fed edge items on a third.  A third
 // stream for the x-slab kind measured slower on C2.
 template <typename T>
 static void launch_sweep(rfb_engine *e, const Args<T> &a, int par) {
+    if (e->plan.tma == 5) {
+        const FusedPlan &p = e->plan;
+        v_launch<T>(a, p.v, p.d_v, p.n_v, e->vmaps[e->nbuf == 2 ? par : 0], e->d_err, e->stream);
+        return;
+    }
     const bool third = edge_on_third_stream(e);
     cudaEventRecord(e->ev_fork, e->stream);
     cudaStreamWaitEvent(e->stream2, e->ev_fork, 0);
@@ -901,10 +935,13 @@ static void launch_dft_run(rfb_engine *e, int count) {
                                              e->n_freqs, e->d_run_omega, e->g.dt, e->dft_t_off, e->d_acc);
 }
 
+static int sweep_launches(const rfb_engine *e) {
+    const FusedPlan &p = e->plan;
+    return p.tma == 5 ? 1 : (p.n_int > 0) + (p.n_edge > 0) + (p.n_qe > 0) + (p.n_qx > 0);
+}
+
 static int count_step_launches(const rfb_engine *e) {
-    int n = (e->sched == RFB_SCHED_FUSED)
-                ? (e->plan.n_int > 0) + (e->plan.n_edge > 0) + (e->plan.n_qe > 0) + (e->plan.n_qx > 0)
-                : 2;
+    int n = e->sched == RFB_SCHED_FUSED ? sweep_launches(e) : 2;
     n += list_launches(e);
     if (e->tf_on) n += 2 + (e->tf_n_h > 0);
     if (e->n_planes) n++;
@@ -940,8 +977,10 @@ static void free_plan_lists(FusedPlan &p) {
     dfree(p.d_edge);
     dfree(p.d_qe);
     dfree(p.d_qx);
+    dfree(p.d_v);
     p.d_int = p.d_edge = p.d_qe = p.d_qx = nullptr;
-    p.n_int = p.n_edge = p.n_qe = p.n_qx = 0;
+    p.d_v = nullptr;
+    p.n_int = p.n_edge = p.n_qe = p.n_qx = p.n_v = p.n_v_plain = 0;
 }
 
 // ---- tensor maps of the TMA interior sweep -----------------------------------
@@ -1023,9 +1062,9 @@ static bool q_fits(const rfb_engine *e) {
     const long long plane = (long long)(g.ny + 1) * e->pitch;
     if (plane >= lim) return false;
     if (!e->cpml.on) return true;
-    const long long x = (long long)e->cpml.eh[0].ns * plane, xm = (long long)e->cpml.em[0].ns * plane;
-    const long long y = (long long)(g.nx + 1) * std::max(e->cpml.eh[1].ns, e->cpml.em[1].ns) * e->pitch;
-    const long long z = (long long)(g.nx + 1) * (g.ny + 1) * std::max(e->cpml.eh[2].ns, e->cpml.em[2].ns);
+    const long long x = (long long)e->cpml.eh[0].slots * plane, xm = (long long)e->cpml.em[0].slots * plane;
+    const long long y = (long long)(g.nx + 1) * std::max(e->cpml.eh[1].slots, e->cpml.em[1].slots) * e->pitch;
+    const long long z = (long long)(g.nx + 1) * (g.ny + 1) * std::max(e->cpml.eh[2].slots, e->cpml.em[2].slots);
     return x < lim && xm < lim && y < lim && z < lim;
 }
 
@@ -1186,8 +1225,260 @@ static void plan_items(const rfb_engine *e, int active, int tj, int tma, int seg
     });
 }
 
+// ---- the vector sweep's plan (mode 5) -----------------------------------------
+// Tile of tr rows x nv vectors: threads, shared-memory layout.  False where
+// the shape exceeds a CTA or a tensor box.
+template <typename T>
+static bool v_layout(VShape &s, int nv, int tr, int wrap, int cj, int ck, bool cpml, bool codes, int nt) {
+    s.nv = nv;
+    s.tr = tr;
+    s.nt = std::max(nt, (int)round_up((long long)(tr + 1) * (nv + 1), 32));
+    s.wrap = wrap;
+    s.cj = cj;
+    s.ck = ck;
+    s.nz = 0x8000000080000000ull;
+    if (nv < 1 || tr < 1 || s.nt > V_NT || (nv + 2) * V_CELLS<T> > 256) return false;
+    s.ebox = 16 * (nv + 2) * (tr + 2);
+    s.hbox = 16 * (nv + 1) * (tr + 1);
+    s.erow = (int)round128(3 * (size_t)s.ebox);
+    s.hrow = (int)round128(3 * (size_t)s.hbox);
+    s.ewrap = (int)round128(48 * (size_t)(nv + 2));
+    s.estage = s.erow + (wrap ? 2 * s.ewrap : 0);
+    s.hstage = s.hrow + (wrap ? (int)round128(48 * (size_t)(nv + 1)) : 0);
+    s.o_rows = v_h_stage(s, V_NH);
+    s.o_last = s.o_rows + 4 * 16 * s.nt;
+    s.o_psi = s.o_last + 4 * (int)sizeof(T) * s.nt;
+    s.o_pz = s.o_psi + (cpml ? 12 * 16 * s.nt : 0);
+    s.o_py = s.o_pz + (cpml ? 6 * 16 * (nv + 1) : 0);
+    s.o_tab = s.o_py + (cpml ? (int)round_up(6 * sizeof(T) * (tr + 1), 16) : 0);
+    s.smem = s.o_tab + (codes ? 512 * (int)sizeof(T) : 0);
+    return s.smem <= V_SMEM;
+}
+// nt: threads of the launch, where it is wider than the tile (a batch)
+static bool v_layout(const rfb_engine *e, VShape &s, int nv, int tr, int cj, int ck, int nt = 0) {
+    const int wrap = (e->g.periodic & 2u) ? 1 : 0;
+    const bool cpml = e->cpml.on != 0, codes = e->scene.codes != nullptr;
+    return e->prec == RFB_FP64 ? v_layout<double>(s, nv, tr, wrap, cj, ck, cpml, codes, nt)
+                               : v_layout<float>(s, nv, tr, wrap, cj, ck, cpml, codes, nt);
+}
+
+// The vector sweep reads no wrapped k column (grids periodic in z run on the
+// scalar sweeps) and counts bytes of psi and codes, and of an item's output
+// planes, by 32 bits.
+static bool v_fits(const rfb_engine *e) {
+    const long long lim = 1LL << 32;
+    const rfb_geom_t &g = e->g;
+    const long long esz = (long long)e->esz, plane = (long long)(g.ny + 1) * e->pitch;
+    if ((g.periodic & 4u) || plane * esz * 8 >= lim || (long long)(g.nx + 1) * plane >= lim) return false;
+    if (!e->cpml.on) return true;
+    const SlabExt *h = e->cpml.eh, *m = e->cpml.em;
+    return (long long)std::max(h[0].slots, m[0].slots) * plane * esz < lim &&
+           (long long)(g.nx + 1) * std::max(h[1].slots, m[1].slots) * e->pitch * esz < lim &&
+           (long long)(g.nx + 1) * (g.ny + 1) * std::max(h[2].slots, m[2].slots) * esz < lim;
+}
+// planes an item may have: its output offsets count bytes from its first plane
+static int v_max_seg(const rfb_engine *e) {
+    const long long plane = (long long)(e->g.ny + 1) * e->pitch * (long long)e->esz;
+    return (int)std::min<long long>(((1LL << 32) - 1) / plane - 1, 1 << 20);
+}
+
+// Tile shape and segment length.  A CTA takes about the same time a plane
+// however small its tile (the plane's chain of dependent instructions, 1.1-
+// 1.4 us on B200), so the rule minimises the planes the busiest CTA slot
+// marches, one more than its length per item: segments that give one wave of
+// CTAs where that takes at most 16 planes each (small grids), else two waves
+// or more of at most 32 planes, which balance the slab items; of all shapes,
+// the one whose march, weighted with its halo threads, is shortest.  Against
+// 24 shapes a grid, on 18 grids of 48^3-256^3, odd extents and both
+// precisions, the rule's pick is on average 3 % and at most 11 % slower than
+// the fastest.
+constexpr int V_REGS = 168;  // registers a thread of k_vsweep holds at most
+
+struct VPick {
+    int tr, nv, seg_int, seg_edge;
+};
+
+static int v_slots(int nt, int smem) {
+    return std::max(1, std::min(65536 / (V_REGS * nt), 227 * 1024 / (smem + 1024)));
+}
+
+// The planes of a tile outside the x slabs and x boundaries: [*xa, *xb).
+static void v_x_range(const rfb_engine *e, int *xa, int *xb) {
+    const rfb_geom_t &g = e->g;
+    const bool on = e->cpml.on != 0, px = g.periodic & 1u;
+    int xlo, xhi;
+    interior_axis(on ? e->cpml.eh[0].lo : 0, on ? e->cpml.eh[0].hi : g.nx, on ? e->cpml.em[0].lo : 0,
+                  on ? e->cpml.em[0].hi : g.nx + 1, g.nx, px, on, &xlo, &xhi);
+    *xa = px ? 0 : xlo + 1;
+    *xb = std::max(*xa, xhi);
+}
+
+static VPick v_rule(const rfb_engine *e, int cj, int ck, int ci) {
+    const int N = e->prec == RFB_FP64 ? 2 : 4, nvk = (ck + N - 1) / N, sms = 148;
+    int xa, xb;
+    v_x_range(e, &xa, &xb);
+    const int len[3] = {std::min(xa, ci), xb - xa, std::max(0, ci - xb)};
+    VPick best = {1, 1, 1, 1};
+    double best_t = 1e300;
+    for (int nk = 1, pv = 0; nk <= nvk; nk++) {
+        const int nv = (nvk + nk - 1) / nk;
+        if (nv == pv) continue;
+        pv = nv;
+        for (int tr = std::min(cj, V_NT / (nv + 1) - 1); tr >= 1; tr--) {
+            const int nj = (cj + tr - 1) / tr;
+            if (tr > 1 && nj == (cj + tr - 2) / (tr - 1)) continue;  // a lower tile does as well
+            VShape s;
+            if (!v_layout(e, s, nv, tr, cj, ck)) continue;
+            const double tiles = (double)((nvk + nv - 1) / nv) * nj, slots = (double)sms * v_slots(s.nt, s.smem);
+            const double per_slot = tiles * ci / slots;
+            const int seg = std::max(1, (int)ceil(per_slot <= 16 ? per_slot : per_slot / std::max(2.0, ceil(per_slot / 32))));
+            double items = 0;
+            for (int q = 0; q < 3; q++) items += tiles * ((len[q] + seg - 1) / seg);
+            const double march = items <= slots ? seg + 1.0 : tiles * ci * (1 + 1.0 / seg) / slots + 0.5 * (seg + 1);
+            // wider halos cost too: half weight on the threads spent per cell
+            const double t = march * (1.0 + (double)(tr + 1) * (nv + 1) / (tr * nv));
+            if (t < best_t) {
+                best_t = t;
+                best = VPick{tr, nv, seg, seg};
+            }
+        }
+    }
+    return best;
+}
+
+// (k, j, i, component) tensor of three consecutive field arrays.
+static int encode_map4(CUtensorMap *m, void *base, CUtensorMapDataType dt, size_t esz, const rfb_geom_t &g,
+                       size_t pitch, size_t field_bytes, unsigned box_w, unsigned box_h) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) {
+        rfb_set_error("the CUDA driver does not provide cuTensorMapEncodeTiled");
+        return -1;
+    }
+    const cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)g.ny + 1, (cuuint64_t)g.nx + 1, 3};
+    const cuuint64_t strides[3] = {(cuuint64_t)(pitch * esz), (cuuint64_t)(pitch * esz * (g.ny + 1)),
+                                   (cuuint64_t)field_bytes};
+    const cuuint32_t box[4] = {box_w, box_h, 1, 3};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    const CUresult r = fn(m, dt, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        rfb_set_error("cuTensorMapEncodeTiled failed (%d)", (int)r);
+        return -1;
+    }
+    return 0;
+}
+
+static int v_encode(rfb_engine *e, const VShape &s) {
+    const CUtensorMapDataType dt =
+        e->prec == RFB_FP64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+    const int N = e->prec == RFB_FP64 ? 2 : 4;
+    const size_t one = e->total * e->esz;
+    for (int par = 0; par < 2; par++) {
+        const int in = e->nbuf == 2 ? par : 0;
+        VMaps &m = e->vmaps[par];
+        void *E = e->fld[in][0], *H = e->fld[in][3];
+        if (encode_map4(&m.e, E, dt, e->esz, e->g, e->pitch, one, (s.nv + 2) * N, s.tr + 2) ||
+            encode_map4(&m.h, H, dt, e->esz, e->g, e->pitch, one, (s.nv + 1) * N, s.tr + 1) ||
+            encode_map4(&m.e1, E, dt, e->esz, e->g, e->pitch, one, (s.nv + 2) * N, 1) ||
+            encode_map4(&m.h1, H, dt, e->esz, e->g, e->pitch, one, (s.nv + 1) * N, 1))
+            return -1;
+    }
+    return 0;
+}
+
+// Items of the shape.  A tile's planes are cut into those outside the x slabs
+// and x boundaries, whose kind names the y / z slabs the tile and its halo
+// touch (0: none, and no boundary either), and the others (V_X).  Items of
+// the same kind together, the costly kinds first.
+static void v_items(const rfb_engine *e, const VShape &s, int ci, int seg_int, int seg_edge, int scene,
+                    std::vector<VItem> &out, int *n_plain) {
+    const rfb_geom_t &g = e->g;
+    const int N = e->prec == RFB_FP64 ? 2 : 4;
+    const bool on = e->cpml.on != 0, py = g.periodic & 2u;
+    int xa, xb;
+    v_x_range(e, &xa, &xb);
+    auto touches = [&](int ax, int q0, int q1) {
+        if (!on) return false;
+        const int n = ax == 1 ? g.ny : g.nz;
+        const SlabExt &h = e->cpml.eh[ax], &m = e->cpml.em[ax];
+        for (int q = std::max(q0, 0); q <= q1; q++) {
+            if (q < n && (q < h.lo || q >= h.hi)) return true;
+            if (q < n + 1 && (q < m.lo || q >= m.hi)) return true;
+        }
+        return false;
+    };
+    std::vector<VItem> kinds[8];
+    auto add = [&](int j0, int k0, int b, int en, int seg, int kind) {
+        // equal segments of at most seg planes
+        const int n = en > b ? (en - b + seg - 1) / seg : 0;
+        for (int q = 0; q < n; q++)
+            kinds[kind].push_back(VItem{j0, k0, b + (int)((long long)(en - b) * q / n),
+                                        b + (int)((long long)(en - b) * (q + 1) / n), kind, scene});
+    };
+    for (int j0 = 0; j0 < s.cj; j0 += s.tr)
+        for (int k0 = 0; k0 < s.ck; k0 += s.nv * N) {
+            const int jl = std::min(j0 + s.tr, s.cj) - 1, kl = std::min(k0 + s.nv * N, (s.ck + N - 1) / N * N) - 1;
+            // a row or vector on a boundary counts as slab (update ranges)
+            const int ky = ((py || j0 >= 1) && jl < g.ny && !touches(1, j0 - 1, jl)) ? 0 : V_Y;
+            const int kz = (k0 >= 1 && kl < g.nz && !touches(2, k0 - 1, kl)) ? 0 : V_Z;
+            if (xb > xa) add(j0, k0, xa, xb, ky | kz ? seg_edge : seg_int, ky | kz);
+            add(j0, k0, 0, std::min(xa, ci), seg_edge, V_X);
+            add(j0, k0, xb, ci, seg_edge, V_X);
+        }
+    *n_plain += (int)kinds[0].size();
+    for (int kind : {(int)V_X, V_Y | V_Z, (int)V_Y, (int)V_Z, 0}) {
+        std::vector<VItem> &v = kinds[kind];
+        std::stable_sort(v.begin(), v.end(), [](const VItem &x, const VItem &y) { return x.ie - x.ib > y.ie - y.ib; });
+        out.insert(out.end(), v.begin(), v.end());
+    }
+}
+
+static void v_extents(const rfb_engine *e, int active, int *cj, int *ck, int *ci) {
+    const rfb_geom_t &g = e->g;
+    *cj = g.ny + ((active && !(g.periodic & 2u)) ? 1 : 0);
+    *ck = g.nz + ((active && !(g.periodic & 4u)) ? 1 : 0);
+    *ci = g.nx + ((active && !(g.periodic & 1u)) ? 1 : 0);
+}
+
+static int v_build_plan(rfb_engine *e, int active, const VPick *pick) {
+    if (!v_fits(e)) {
+        rfb_set_error("sweep mode 5 (vector cells) needs a z axis that is not periodic and psi arrays and code volumes of fewer than 2^32 bytes");
+        return -1;
+    }
+    FusedPlan &p = e->plan;
+    free_plan_lists(p);
+    int cj, ck, ci;
+    v_extents(e, active, &cj, &ck, &ci);
+    const VPick v = pick ? *pick : v_rule(e, cj, ck, ci);
+    if (!v_layout(e, p.v, v.nv, v.tr, cj, ck)) {
+        rfb_set_error("sweep tile of %d rows x %d vectors exceeds a CTA", v.tr, v.nv);
+        return -1;
+    }
+    p.tj = v.tr;
+    p.ns = v.nv;
+    p.tma = 5;
+    p.uni = 1;
+    p.i2 = 0;
+    p.seg_int = std::min(v.seg_int, v_max_seg(e));
+    p.seg_edge = std::min(v.seg_edge, v_max_seg(e));
+    p.d = FusedDims{cj, ck, ci};
+    std::vector<VItem> items;
+    v_items(e, p.v, ci, p.seg_int, p.seg_edge, 0, items, &p.n_v_plain);
+    p.n_v = (int)items.size();
+    CK(dmalloc(&p.d_v, items.size() * sizeof(VItem)));
+    CK(cudaMemcpy(p.d_v, items.data(), items.size() * sizeof(VItem), cudaMemcpyHostToDevice));
+    return v_encode(e, p.v);
+fail:
+    return -1;
+}
+
 static int build_sweep_plan(rfb_engine *e, int active, int tj, int ns, int tma, int seg_int, int seg_edge,
                             int uni = 0, int i2 = 0) {
+    if (tma == 5) {
+        const VPick v = {tj, ns, seg_int, seg_edge};
+        return v_build_plan(e, active, &v);
+    }
     if (i2 && (tma < 2 || uni || e->prec != RFB_FP32 || tj != 8 || (i2 != 3 && i2 != 4))) {
         rfb_set_error("the two-rows interior sweep needs an FP32 plan of mode 2 or 3, three launches, 8-row tiles "
                       "and ring depth 3 or 4");
@@ -1255,7 +1546,8 @@ fail:
 static bool plan_variant_known(int prec, int tj, int ns, int tma) {
     const InteriorVariant *v;
     size_t n;
-    if (tma < 0 || tma > 4) return false;
+    if (tma < 0 || tma > 5) return false;
+    if (tma == 5) return tj >= 1 && ns >= 1;  // any shape that fits a CTA
     if (tma >= 2) {
         v = prec == RFB_FP32 ? kQVariantsFp32 : kQVariantsFp64;
         n = prec == RFB_FP32 ? std::size(kQVariantsFp32) : std::size(kQVariantsFp64);
@@ -1421,7 +1713,8 @@ extern "C" void rfb_engine_destroy(rfb_engine_t *e) {
     dfree(e->d_run_omega);
     dfree(e->d_acc);
     dfree(e->d_omega); dfree(e->d_re); dfree(e->d_im);
-    dfree(e->plan.d_int); dfree(e->plan.d_edge); dfree(e->plan.d_qe); dfree(e->plan.d_qx); dfree(e->plan.d_queue);
+    free_plan_lists(e->plan);
+    dfree(e->plan.d_queue);
     dfree(e->tf_inc_e); dfree(e->tf_inc_h); dfree(e->tf_src); dfree(e->tf_h_cell); dfree(e->tf_h_comp);
     dfree(e->tf_h_first); dfree(e->tf_h_count); dfree(e->tf_h_idx); dfree(e->tf_h_coef); dfree(e->tf_h_w);
     dfree(e->tf_e_first); dfree(e->tf_e_count); dfree(e->tf_e_idx); dfree(e->tf_e_coef);
@@ -1597,7 +1890,8 @@ static rfb_engine_t *engine_create(const rfb_geom_t *geom, int precision, int sc
         e->active = active;
         if (member) {
             // a batch scene: the batch builds the plans and owns the streams
-            if (tma_prepare() != 0 || q_prepare() != 0 || qi2_prepare() != 0) {
+            if (tma_prepare() != 0 || q_prepare() != 0 || qi2_prepare() != 0 || v_prepare<float>() != 0 ||
+                v_prepare<double>() != 0) {
                 rfb_set_error("cannot configure the TMA sweep kernels' shared memory");
                 goto fail_noset;
             }
@@ -1608,7 +1902,8 @@ static rfb_engine_t *engine_create(const rfb_geom_t *geom, int precision, int sc
         CK(cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&e->ev_join3, cudaEventDisableTiming));
-        if (tma_prepare() != 0 || q_prepare() != 0 || qi2_prepare() != 0) {
+        if (tma_prepare() != 0 || q_prepare() != 0 || qi2_prepare() != 0 || v_prepare<float>() != 0 ||
+            v_prepare<double>() != 0) {
             rfb_set_error("cannot configure the TMA sweep kernels' shared memory");
             goto fail_noset;
         }
@@ -1622,6 +1917,8 @@ static rfb_engine_t *engine_create(const rfb_geom_t *geom, int precision, int sc
         if (nov >= 4 && a3 > 0 && a4 > 0 && plan_variant_known(precision, a1, a2, nov >= 5 ? a5 : 0) &&
             (a6 == 0 || (a6 == 1 && a5 >= 2)))
             rc = build_sweep_plan(e, active, a1, a2, nov >= 5 ? a5 : 0, a3, a4, a6, a7);
+        else if (!ov && v_fits(e))
+            rc = v_build_plan(e, active, nullptr);
         else if (ov)
             rc = (rfb_set_error("sweep plan \"%s\" names no sweep variant", ov), -1);
         else if (!rfb_tune_enabled())
@@ -1838,8 +2135,8 @@ extern "C" int rfb_engine_info(rfb_engine_t *e, rfb_engine_info_t *out) {
     out->unified = e->plan.uni;
     out->interior_ring2 = e->plan.i2;
     out->seg_edge = e->plan.seg_edge;
-    out->interior_items = e->plan.n_int;
-    out->edge_items = e->plan.n_edge + e->plan.n_qe + e->plan.n_qx;
+    out->interior_items = e->plan.n_int + e->plan.n_v_plain;
+    out->edge_items = e->plan.n_edge + e->plan.n_qe + e->plan.n_qx + e->plan.n_v - e->plan.n_v_plain;
     size_t sca = 0;
     if (e->cpml.on) {
         // cells of the swept volume inside the slab of each axis (H profiles)
@@ -1868,7 +2165,7 @@ static int time_kernels_t(rfb_engine *e, size_t n, double *sweep_ms, double *oth
         CK(cudaEventRecord(ev[0], e->stream));
         if (e->sched == RFB_SCHED_FUSED) {
             launch_sweep<T>(e, a, par);
-            g_launches += (e->plan.n_int > 0) + (e->plan.n_edge > 0) + (e->plan.n_qe > 0) + (e->plan.n_qx > 0);
+            g_launches += sweep_launches(e);
         } else {
             dim3 blk(32, 8), grd((g.nz + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nx + 1);
             k_h_split<T><<<grd, blk, 0, e->stream>>>(a);

@@ -45,6 +45,32 @@ struct SweepItem {
     int sub = 0;
 };
 
+// Tile shape and shared-memory layout of the vector sweep (vsweep.cuh),
+// computed by the host.
+struct VShape {
+    int nv, tr;            // own vectors per row, own rows per tile
+    int nt;                // threads: (tr + 1)(nv + 1) rounded up to warps
+    int wrap;              // periodic y: one-row boxes follow the tile's
+    int ebox, hbox;        // bytes of a component's box in a stage
+    // periodic y: offsets in a stage of the wrapped rows ny - 1 (E, H) and,
+    // ewrap bytes after it, 0 (E), three components each
+    int erow, hrow, ewrap;
+    int estage, hstage;    // bytes of a stage
+    int cj, ck;            // covered extents
+    int o_rows, o_last, o_psi, o_py, o_pz, o_tab;  // offsets in shared memory (vsweep.cuh)
+    int smem;              // dynamic shared memory of the CTA
+    unsigned long long nz; // -0 in both FP32 halves (see vm in vsweep.cu)
+};
+
+// its work items: kind 0 (no slab, no boundary) or the slabs touched (bits;
+// an item with V_X may touch any, a boundary item names at least one), a
+// batch's scene
+enum { V_Z = 1, V_Y = 2, V_X = 4 };
+struct VItem {
+    int j0, k0, ib, ie;
+    int kind, scene;
+};
+
 struct FusedPlan {
     int tj = 8, ns = 6;   // interior variant (rows per tile, ring depth)
     // interior planes staged per thread by cp.async (0), by the TMA (1), or
@@ -66,6 +92,10 @@ struct FusedPlan {
     int n_qe = 0, n_qx = 0;                         // modes 2, 3: edge and x-slab items of k_sweep_q
     SweepItem *d_qe = nullptr, *d_qx = nullptr;
     int *d_queue = nullptr;                         // counters (interior 0-1, edge 2-3, x slab 4-5)
+    // mode 5: the vector sweep (vsweep.cuh) over every item in one launch
+    VShape v;
+    VItem *d_v = nullptr;
+    int n_v = 0, n_v_plain = 0;
 };
 
 template <typename T>
@@ -319,9 +349,9 @@ __device__ __forceinline__ void prof_at(const T *kinv, const T *b, const T *ac, 
 }
 
 // Slab index of q, -1 in the unstretched interior or outside [0, len).
-__device__ __forceinline__ int slab_in(int q, int lo, int hi, int len, int on) {
+__device__ __forceinline__ int slab_in(int q, int lo, int hi, int off, int len, int on) {
     if (!on || q < 0 || q >= len) return -1;
-    return slab_of(q, lo, hi);
+    return slab_of(q, lo, hi, off);
 }
 
 // Per-CTA profile tables in shared memory.
@@ -389,22 +419,22 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
     }
     // slab indices of the own cell (H side: q < n; E side: only swept samples
     // use them, and those have q < n)
-    const int sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.ny, on);
-    const int skh = slab_in(k, a.lo_h[2], a.hi_h[2], a.nz, on);
-    const int sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.ny, on);
-    const int skm = slab_in(k, a.lo_m[2], a.hi_m[2], a.nz, on);
+    const int sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+    const int skh = slab_in(k, a.lo_h[2], a.hi_h[2], a.off_h[2], a.nz, on);
+    const int sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.off_m[1], a.ny, on);
+    const int skm = slab_in(k, a.lo_m[2], a.hi_m[2], a.off_m[2], a.nz, on);
     // halo cells: row (j0-1, k) for warp 0, column (j0+tx, k0-1) for warp 1
-    const int sjh_row = slab_in(j0 - 1, a.lo_h[1], a.hi_h[1], a.ny, on);
+    const int sjh_row = slab_in(j0 - 1, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
     const int jc = j0 + tx;
-    const int sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.ny, on);
-    const int skh_col = slab_in(k0 - 1, a.lo_h[2], a.hi_h[2], a.nz, on);
+    const int sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+    const int skh_col = slab_in(k0 - 1, a.lo_h[2], a.hi_h[2], a.off_h[2], a.nz, on);
     const int nshy = a.ns_h[1], nshz = a.ns_h[2], nsmy = a.ns_m[1], nsmz = a.ns_m[2];
 
     // psi copies of plane p into stage st
     auto issue_psi = [&](EdgeStage<T, TJ> &st, int p) {
         if (!on || p < 0) return;
-        const int sxh = slab_in(p, a.lo_h[0], a.hi_h[0], a.nx, on);
-        const int sxm = slab_in(p, a.lo_m[0], a.hi_m[0], a.nx, on);
+        const int sxh = slab_in(p, a.lo_h[0], a.hi_h[0], a.off_h[0], a.nx, on);
+        const int sxm = slab_in(p, a.lo_m[0], a.hi_m[0], a.off_m[0], a.nx, on);
         if (own) {
             if (sjh >= 0) {
                 const long long o = ((long long)p * nshy + sjh) * a.pitch + k;
@@ -481,7 +511,7 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
                       const EdgeStage<T, TJ> &cs, const EdgeStage<T, TJ> &ns, bool store) -> T {
         const FusedStage<T, TJ> &cur = cs.f, &nxt = ns.f;
         const T hin = cur.h[c][rr][qq];
-        const int sx = slab_in(i, a.lo_h[0], a.hi_h[0], a.nx, on);
+        const int sx = slab_in(i, a.lo_h[0], a.hi_h[0], a.off_h[0], a.nx, on);
         T dA, dB;
         if (c == 0) {
             if (!(i < a.nx + (px ? 0 : 1) && jj < a.ny && kk < a.nz)) return hin;
@@ -599,7 +629,7 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
             }
             if (!skip) {
                 const T ca = s_tab[code], cb = s_tab[256 + code];
-                const int sxm = slab_in(i, a.lo_m[0], a.hi_m[0], a.nx, on);
+                const int sxm = slab_in(i, a.lo_m[0], a.hi_m[0], a.off_m[0], a.nx, on);
                 if (e_updated(a, 0, i, j, k)) {
                     T tA = xs(sH[2][r][q], sH[2][r - 1][q]);
                     T tB = xs(sH[1][r][q], sH[1][r][q - 1]);

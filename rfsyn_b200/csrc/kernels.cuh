@@ -61,8 +61,10 @@ struct Args {
     int cpml_on;
     const T *kinv_m[3], *b_m[3], *a_m[3];
     const T *kinv_h[3], *b_h[3], *a_h[3];
-    int lo_m[3], hi_m[3], ns_m[3];
-    int lo_h[3], hi_h[3], ns_h[3];
+    // slab cells of each axis: [0, lo) and [hi, ..), at slots q and q + off of
+    // a psi array whose slab axis holds ns slots
+    int lo_m[3], hi_m[3], ns_m[3], off_m[3];
+    int lo_h[3], hi_h[3], ns_h[3], off_h[3];
     T *psi_e[6];
     T *psi_hi[6], *psi_ho[6];
     // scene
@@ -102,11 +104,11 @@ __device__ __forceinline__ long long cidx(const Args<T> &a, int i, int j, int k)
     return ((long long)i * (a.ny + 1) + j) * a.pitch + k;
 }
 
-__device__ __forceinline__ int slab_of(int q, int lo, int hi) {
-    return q < lo ? q : (q >= hi ? lo + (q - hi) : -1);
+__device__ __forceinline__ int slab_of(int q, int lo, int hi, int off) {
+    return q < lo ? q : (q >= hi ? q + off : -1);
 }
 
-// Index of slab cell s of a psi array whose slab axis is `axis`.
+// Index of slab slot s of a psi array whose slab axis is `axis`.
 template <typename T>
 __device__ __forceinline__ long long psi_idx(const Args<T> &a, int axis, int ns, int s, int i, int j, int k) {
     if (axis == 0) return ((long long)s * (a.ny + 1) + j) * a.pitch + k;
@@ -128,7 +130,7 @@ __device__ __forceinline__ T cpml_step(T diff, T kinv, T b, T ac, T dx, T psi_ol
 template <typename T>
 __device__ __forceinline__ T h_term(const Args<T> &a, int p, int axis, int q, T diff, int i, int j, int k) {
     if (!a.cpml_on) return diff;
-    int s = slab_of(q, a.lo_h[axis], a.hi_h[axis]);
+    int s = slab_of(q, a.lo_h[axis], a.hi_h[axis], a.off_h[axis]);
     if (s < 0) return diff;
     long long pi = psi_idx(a, axis, a.ns_h[axis], s, i, j, k);
     T pn;
@@ -140,7 +142,7 @@ __device__ __forceinline__ T h_term(const Args<T> &a, int p, int axis, int q, T 
 template <typename T>
 __device__ __forceinline__ T e_term(const Args<T> &a, int p, int axis, int q, T diff, int i, int j, int k) {
     if (!a.cpml_on) return diff;
-    int s = slab_of(q, a.lo_m[axis], a.hi_m[axis]);
+    int s = slab_of(q, a.lo_m[axis], a.hi_m[axis], a.off_m[axis]);
     if (s < 0) return diff;
     long long pi = psi_idx(a, axis, a.ns_m[axis], s, i, j, k);
     T pn;
@@ -769,7 +771,7 @@ __global__ void k_probe_dft(const T *ts, long long n_steps, int n_probes, int st
 }
 
 // Marks list cells in a code volume (code-less scenes with many list cells).
-__global__ void k_mark_list(uint8_t *codes, const int *ijk, int n, int ny, long long pitch) {
+static __global__ void k_mark_list(uint8_t *codes, const int *ijk, int n, int ny, long long pitch) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     codes[((long long)ijk[3 * q] * (ny + 1) + ijk[3 * q + 1]) * pitch + ijk[3 * q + 2]] = LIST_CODE;

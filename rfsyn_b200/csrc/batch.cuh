@@ -104,9 +104,11 @@ __global__ void __launch_bounds__(32 * TJ, MINB)
 template <typename T>
 __global__ void __launch_bounds__(256) k_e_list_b(const Args<T> *args, const int2 *blocks) {
     __shared__ Args<T> sa;
+    grid_launch_next();
     const int2 b = blocks[blockIdx.x];
     load_args(sa, args + b.x, 256, threadIdx.x);
     __syncthreads();
+    grid_wait();
     const int e = b.y + threadIdx.x;
     if (e < 3 * sa.n_cells) e_list_entry(sa, e);
 }
@@ -123,6 +125,8 @@ struct ProbeRefB {
 template <typename T>
 __global__ void k_probe_gather_b(const ProbeRefB<T> *p, int n, int out_buf, long long n_steps, int *d_step) {
     __shared__ int step;
+    grid_launch_next();
+    grid_wait();
     if (threadIdx.x == 0) step = *d_step;
     __syncthreads();
     if (step < n_steps)
@@ -225,6 +229,7 @@ struct rfb_batch {
     BatchItem *d_items[3] = {};    // interior, x slab, edge (uni: every item in the edge list)
     int n_items[3] = {};
     int uni = 0;
+    bool overlap = false;          // launches are being captured as programmatic dependents
     // mode 5: the vector sweep's items of every scene, shapes and maps
     VItem *d_vitems = nullptr;
     int n_vitems = 0, n_vplain = 0, v_nt = 0, v_smem = 0;
@@ -435,7 +440,7 @@ static void batch_sweep(rfb_batch *b, int par) {
     const Args<T> *args = (const Args<T> *)b->d_args[par];
     if (b->mode == 5) {
         v_launch_b<T>(args, b->d_vshapes, b->d_vmaps[par], b->d_vitems, b->n_vitems, b->v_nt, b->v_smem, b->d_err,
-                      b->stream);
+                      b->stream, b->overlap);
         return;
     }
     const TmaMaps *maps = b->d_maps[par];
@@ -459,9 +464,10 @@ static void batch_sweep(rfb_batch *b, int par) {
 template <typename T>
 static void batch_rest(rfb_batch *b, int par) {
     if (b->n_lblocks)
-        k_e_list_b<T><<<b->n_lblocks, 256, 0, b->stream>>>((const Args<T> *)b->d_args[par], b->d_lblocks);
-    k_probe_gather_b<T><<<1, 1024, 0, b->stream>>>((const ProbeRefB<T> *)b->d_probes, b->n_probes, 1 - par,
-                                                   (long long)b->n_steps, b->d_step);
+        launch_step(k_e_list_b<T>, dim3(b->n_lblocks), dim3(256), 0, b->stream, b->overlap,
+                    (const Args<T> *)b->d_args[par], b->d_lblocks);
+    launch_step(k_probe_gather_b<T>, dim3(1), dim3(1024), 0, b->stream, b->overlap,
+                (const ProbeRefB<T> *)b->d_probes, b->n_probes, 1 - par, (long long)b->n_steps, b->d_step);
 }
 
 static int batch_launches_per_step(const rfb_batch *b) {
@@ -483,10 +489,12 @@ static int batch_graph(rfb_batch *b, int par, int steps, cudaGraphExec_t *out) {
     cudaGraph_t graph = nullptr;
     int p = par;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    b->overlap = b->mode == 5 && b->cells <= (1 << 21) && 3 * b->list_cells <= (1 << 17);  // as overlap_pays
     for (int s = 0; s < steps; s++) {
         batch_enqueue_step(b, p);
         p ^= 1;
     }
+    b->overlap = false;
     CK(cudaStreamEndCapture(b->stream, &graph));
     CK(cudaGraphInstantiate(out, graph, 0));
     cudaGraphDestroy(graph);

@@ -12,6 +12,36 @@
 
 namespace rfb {
 
+// ---- kernels of a step overlap their launches ---------------------------------
+// A small scene's step is a chain of short kernels, and each link costs the
+// launch and the drain of the kernel before it (~2 us on B200).  Inside the
+// step graphs the links are programmatic: a kernel's CTAs start once every
+// CTA of the kernel before it has started (grid_launch_next, first thing in
+// each kernel) and do what reads no other kernel's results; grid_wait then
+// holds them until that kernel has ended and its writes are visible.  Every
+// CTA of every step kernel passes grid_wait, also one without work, so the
+// kernels' ends keep their order.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches a step kernel, with overlap as a programmatic dependent of the
+// kernel before it in the stream.
+template <typename... P, typename... A>
+static inline void launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool overlap,
+                               const A &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = overlap ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double xa(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double xs(double a, double b) { return __dsub_rn(a, b); }
@@ -501,6 +531,8 @@ struct TfArgs {
 // each of their terms, in order (E1D at step n).
 template <typename T>
 __global__ void k_tfsf_h(TfArgs<T> a) {
+    grid_launch_next();
+    grid_wait();
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.n_h) return;
     T *f = a.Ho[a.h_comp[q]] + a.h_cell[q];
@@ -515,6 +547,8 @@ __global__ void k_tfsf_h(TfArgs<T> a) {
 // The line's H: H1D[m] -= ch (E1D[m+1] - E1D[m]).
 template <typename T>
 __global__ void k_inc_h(TfArgs<T> a) {
+    grid_launch_next();
+    grid_wait();
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < a.m_len - 1; m += gridDim.x * blockDim.x)
         a.inc_h[m] = xs(a.inc_h[m], xm(a.ch, xs(a.inc_e[m + 1], a.inc_e[m])));
 }
@@ -523,6 +557,8 @@ __global__ void k_inc_h(TfArgs<T> a) {
 // of the step just completed (the step counter already advanced).
 template <typename T>
 __global__ void k_inc_e(TfArgs<T> a) {
+    grid_launch_next();
+    grid_wait();
     for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < a.m_len - 1; m += gridDim.x * blockDim.x) {
         if (m == 0) {
             const long long n = *a.d_step;
@@ -535,6 +571,8 @@ __global__ void k_inc_e(TfArgs<T> a) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_e_list(Args<T> a) {
+    grid_launch_next();
+    grid_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (a.l_work) {
         if (t < a.n_work) e_list_entry(a, a.l_work[t]);
@@ -558,6 +596,8 @@ __global__ void __launch_bounds__(256) k_e_list(Args<T> a) {
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 3) k_list_cells(Args<T> a, const int *t3, int n_t3, int nb_t3, const int *ade,
                                                     int n_ade, int nb_ade) {
+    grid_launch_next();
+    grid_wait();
     const int b = blockIdx.x;
     if (b < nb_t3) {
         const int t = b * blockDim.x + threadIdx.x;
@@ -588,6 +628,8 @@ struct ProbeArgs {
 template <typename T>
 __global__ void k_probe_gather(ProbeArgs<T> p) {
     __shared__ int n;
+    grid_launch_next();
+    grid_wait();
     if (threadIdx.x == 0) n = *p.d_step;
     __syncthreads();
     if (n < p.n_steps)
@@ -622,6 +664,8 @@ __global__ void __launch_bounds__(kPlaneThreads) k_plane_gather(const PlaneDesc 
                                                                 long long n_steps, const int *d_step, double *part,
                                                                 int *count, int max_chunks) {
     __shared__ double warp_sum[kPlaneThreads / 32];
+    grid_launch_next();
+    grid_wait();
     const int q = blockIdx.y, b = blockIdx.x;
     if (q >= n_planes) return;
     const int n = *d_step;
@@ -672,6 +716,8 @@ __global__ void __launch_bounds__(kPlaneThreads) k_plane_gather(const PlaneDesc 
 template <typename T>
 __global__ void k_dft_run(const T *ts, int n_series, long long n_steps, const int *d_step, int count, int n_freqs,
                           const double *omega, double dt, double t_off, void *acc) {
+    grid_launch_next();
+    grid_wait();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     const int p = blockIdx.y;
     if (f >= n_freqs || p >= n_series) return;

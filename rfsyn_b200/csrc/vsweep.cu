@@ -259,9 +259,6 @@ __device__ __forceinline__ bool v_item(const Args<T> &a, const VShape &sh, const
         load_e(eslot, plane_of(n + 1), bar);
         load_h(hslot, plane_of(n), bar);
     };
-    int issued = 0;
-    if (tid == 0)
-        for (; issued < V_NH && issued <= steps; issued++) issue(issued, issued + 1, issued);
 
     // ---- the thread's vector ----
     const int rr = tid / nv1, vv = tid - rr * nv1;
@@ -460,6 +457,12 @@ __device__ __forceinline__ bool v_item(const Args<T> &a, const VShape &sh, const
         }
         cp_async_commit();
     };
+    // everything so far reads only what no step writes; from here on the
+    // fields and psi of the launches before this one
+    grid_wait();
+    int issued = 0;
+    if (tid == 0)
+        for (; issued < V_NH && issued <= steps; issued++) issue(issued, issued + 1, issued);
     int i = plane_of(0);
     // groups of a thread's copies alternate H psi, E psi: each wait below
     // leaves the newest one in flight
@@ -753,6 +756,7 @@ __device__ __forceinline__ bool v_run(const Args<T> &a, const VShape &sh, const 
 __device__ __forceinline__ bool v_begin(unsigned char *smem, int *err) {
     if (__cvta_generic_to_shared(smem) & 127u) {
         if (threadIdx.x == 0) atomicExch(err, 2);
+        grid_wait();
         return false;
     }
     if (threadIdx.x == 0) {
@@ -769,6 +773,7 @@ __global__ void __launch_bounds__(V_NT, V_MB)
     k_vsweep(const __grid_constant__ Args<T> a, const __grid_constant__ VShape sh, const VItem *items,
              const __grid_constant__ VMaps maps, int *err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    grid_launch_next();
     if (!v_begin(smem_raw, err)) return;
     const VItem it = items[blockIdx.x];
     if (!v_run<T>(a, sh, maps, it, smem_raw) && threadIdx.x == 0) atomicExch(err, 1);
@@ -783,6 +788,7 @@ __global__ void __launch_bounds__(V_NT, V_MB)
     k_vsweep_b(const Args<T> *args, const VShape *shapes, const VMaps *maps, const VItem *items, int args_off,
                int *err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
+    grid_launch_next();
     const VItem it = items[blockIdx.x];
     Args<T> &sa = *reinterpret_cast<Args<T> *>(smem_raw + args_off);
     VShape &sh = *reinterpret_cast<VShape *>(smem_raw + args_off + (sizeof(Args<T>) + 15) / 16 * 16);
@@ -816,26 +822,27 @@ int v_prepare() {
 
 template <typename T>
 void v_launch(const Args<T> &a, const VShape &sh, const VItem *items, int n, const VMaps &maps, int *err,
-              cudaStream_t st) {
-    if (n > 0) k_vsweep<T><<<n, sh.nt, sh.smem, st>>>(a, sh, items, maps, err);
+              cudaStream_t st, bool overlap) {
+    if (n > 0) launch_step(k_vsweep<T>, dim3(n), dim3(sh.nt), sh.smem, st, overlap, a, sh, items, maps, err);
 }
 
 template <typename T>
 void v_launch_b(const Args<T> *args, const VShape *shapes, const VMaps *maps, const VItem *items, int n, int nt,
-                int smem, int *err, cudaStream_t st) {
+                int smem, int *err, cudaStream_t st, bool overlap) {
     if (n > 0)
-        k_vsweep_b<T><<<n, nt, smem + v_args_bytes<T>(), st>>>(args, shapes, maps, items, smem, err);
+        launch_step(k_vsweep_b<T>, dim3(n), dim3(nt), smem + v_args_bytes<T>(), st, overlap, args, shapes, maps, items,
+                    smem, err);
 }
 
 template int v_prepare<float>();
 template int v_prepare<double>();
 template void v_launch<float>(const Args<float> &, const VShape &, const VItem *, int, const VMaps &, int *,
-                              cudaStream_t);
+                              cudaStream_t, bool);
 template void v_launch<double>(const Args<double> &, const VShape &, const VItem *, int, const VMaps &, int *,
-                               cudaStream_t);
+                               cudaStream_t, bool);
 template void v_launch_b<float>(const Args<float> *, const VShape *, const VMaps *, const VItem *, int, int, int,
-                                int *, cudaStream_t);
+                                int *, cudaStream_t, bool);
 template void v_launch_b<double>(const Args<double> *, const VShape *, const VMaps *, const VItem *, int, int, int,
-                                 int *, cudaStream_t);
+                                 int *, cudaStream_t, bool);
 
 }  // namespace rfb

@@ -73,12 +73,12 @@ __host__ __device__ __forceinline__ int v_h_stage(const VShape &s, int q) {
 }
 
 // Host entry points (vsweep.cu): shared memory limits of the kernels; one
-// launch of the sweep over n items.
+// launch of the sweep over n items (overlap: see launch_step).
 template <typename T>
 int v_prepare();
 template <typename T>
 void v_launch(const Args<T> &a, const VShape &sh, const VItem *items, int n, const VMaps &maps, int *err,
-              cudaStream_t st);
+              cudaStream_t st, bool overlap);
 // ... over n items of many scenes: CTAs of nt threads, smem bytes for the
 // tile and v_args_bytes behind them for the scene's parameters (smem a
 // multiple of 16).
@@ -88,6 +88,6 @@ constexpr int v_args_bytes() {
 }
 template <typename T>
 void v_launch_b(const Args<T> *args, const VShape *shapes, const VMaps *maps, const VItem *items, int n, int nt,
-                int smem, int *err, cudaStream_t st);
+                int smem, int *err, cudaStream_t st, bool overlap);
 
 }  // namespace rfb

@@ -10,37 +10,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "overlap.cuh"
+
 namespace rfb {
-
-// ---- kernels of a step overlap their launches ---------------------------------
-// A small scene's step is a chain of short kernels, and each link costs the
-// launch and the drain of the kernel before it (~2 us on B200).  Inside the
-// step graphs the links are programmatic: a kernel's CTAs start once every
-// CTA of the kernel before it has started (grid_launch_next, first thing in
-// each kernel) and do what reads no other kernel's results; grid_wait then
-// holds them until that kernel has ended and its writes are visible.  Every
-// CTA of every step kernel passes grid_wait, also one without work, so the
-// kernels' ends keep their order.
-__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// Launches a step kernel, with overlap as a programmatic dependent of the
-// kernel before it in the stream.
-template <typename... P, typename... A>
-static inline void launch_step(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool overlap,
-                               const A &...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = overlap ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
 
 __device__ __forceinline__ double xm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double xa(double a, double b) { return __dadd_rn(a, b); }

@@ -4,24 +4,29 @@
 // parameter vector to its tx -> rx transfer function.
 //
 // Kernels:
-//   k_gemm_nt   C[M,N] = A[M,K] . B[N,K]^T on the tensor cores (BF16 operands,
-//               mma.sync m16n8k16, FP32 accumulation), 64x64 CTA tiles, A/B
-//               tiles staged by cp.async (two stages), fused epilogues: bias +
-//               GELU (hidden layers, pre-activation kept in FP32), bias (output
-//               layer), GELU' (backward through a hidden layer, dZ in FP32,
-//               BF16 and transposed BF16), plain FP32 (weight gradients);
+//   k_gemm      C[M,N] = op(A) op(B) on the tensor cores (BF16 operands,
+//               mma.sync m16n8k16, FP32 accumulation), operands in either
+//               layout, tiles staged by cp.async (four stages), fused
+//               epilogues: bias + GELU (hidden layers, pre-activation kept in
+//               FP32 for the backward pass), bias (output layer), GELU'
+//               (backward through a hidden layer, dZ in FP32 and BF16), plain
+//               FP32 (weight gradients);
 //   k_gemm_tc   the same products and epilogues on tcgen05 (accumulators in
 //               tensor memory), selectable; slower on this network's products;
-//   k_mse       loss gradient 2 (out - y) / (M N), FP32 / BF16 / transposed,
-//               per-block loss partials (deterministic);
+//   k_mse       loss gradient 2 (out - y) / (M N), FP32 / BF16, per-block loss
+//               partials (deterministic);
 //   k_colsum    bias gradients as deterministic column sums of dZ;
-//   k_adam      Adam with bias correction and a cosine learning rate taken
-//               from the device step counter; writes the BF16 weights and
-//               their transposes used by the next step's GEMMs;
+//   k_adam      Adam over every parameter in one launch, with bias correction
+//               and a cosine learning rate taken from the device step
+//               counter; writes the BF16 weights used by the next step's
+//               GEMMs and advances the counter;
 //   k_gather    a training batch from the resident data set through a
 //               per-epoch permutation and the device step counter.
-// One training step is ~8 launches per layer; the whole step is captured in
-// a CUDA graph and replayed.
+// The transposed copies (weights, activations, dZ) exist only for k_gemm_tc,
+// whose operands are both K-major.
+// One training step (gather, forward, loss, backward, Adam) is captured in a
+// CUDA graph and replayed; the weight and bias gradients run beside the chain
+// of dX products on streams of their own.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -33,22 +38,26 @@
 #include <vector>
 
 #include "engine.h"
+#include "overlap.cuh"
 
 typedef __nv_bfloat16 bf16;
+using rfb::grid_launch_next;
+using rfb::grid_wait;
+using rfb::launch_step;
 
 namespace {
 
-constexpr int GT = 64;   // CTA tile (M and N)
-constexpr int GK = 32;   // K per stage
-constexpr int SROW = 40; // shared row length (bf16): 80 bytes, conflict-free fragment loads
+constexpr int GK = 64;      // K per stage
+constexpr int GSTAGES = 4;  // stages of the ring
+constexpr int GRAPH_STEPS = 8;  // training steps of the larger graph
 
 enum { EPI_HIDDEN = 0, EPI_OUT = 1, EPI_BWD_GELU = 2, EPI_F32 = 3 };
 
 struct Epi {
     const float *bias;   // [N] (HIDDEN, OUT)
-    float *f32;          // HIDDEN: pre-activation; OUT: output; BWD_GELU: dZ; F32: C
+    float *f32;          // HIDDEN: pre-activation (or null); OUT: output; BWD_GELU: dZ; F32: C
     bf16 *b16;           // HIDDEN: GELU(pre); BWD_GELU: dZ
-    bf16 *b16t;          // BWD_GELU: dZ^T ([N][M])
+    bf16 *b16t;          // BWD_GELU: dZ^T ([N][M]), or null
     const float *pre;    // BWD_GELU: pre-activation of the layer whose output gradient this is
 };
 
@@ -73,81 +82,123 @@ __device__ __forceinline__ void mma_bf16(float c[4], unsigned a0, unsigned a1, u
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// C = A . B^T.  A: [M][lda] bf16 row-major, B: [N][ldb] bf16 row-major.
-// M, N multiples of 64, K a multiple of 32, lda / ldb multiples of 8.
-template <int EPI>
-__global__ void __launch_bounds__(128) k_gemm_nt(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B,
-                                                 int ldb, int M, int N, int K, Epi epi) {
-    __shared__ __align__(16) bf16 As[2][GT][SROW];
-    __shared__ __align__(16) bf16 Bs[2][GT][SROW];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * GT, n0 = blockIdx.x * GT;
-    float acc[2][4][4] = {};
+// 16-byte chunk c of row r of a tile whose rows hold CH chunks: where it lies,
+// so that the eight rows of an ldmatrix fall on different banks.
+template <int CH>
+__device__ __forceinline__ int swz(int r, int c) {
+    return CH == 8 ? (c ^ (r & 7)) : (c ^ ((r >> 1) & 3));
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(unsigned (&r)[4], unsigned addr) {
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+}
 
+// C = op(A) op(B): A is [M][lda] (K contiguous), with TA [K][lda] (M
+// contiguous); B is [N][ldb], with TB [K][ldb].  M, N multiples of the tile,
+// K of 64, lda / ldb of 8.  BM x BN output tiles, four warps as 2 x 2.
+//
+// Bound by latency: a training step's products are 0.13 GFLOP, so what counts
+// is how many CTAs there are and how far the loads run ahead.  32 x 32 tiles
+// give 256 x 512 outputs 128 CTAs (64 x 64 tiles: 32 on 148 SMs), and three
+// 64-deep stages are in flight while one is used: 4.2-7.2 us a product of
+// the 256-row step, cold, against 6.6-17.1 us with 64 x 64 tiles, two 32-deep
+// stages and scalar fragment loads; the whole step 0.21 -> 0.068 ms with the
+// changes around it.  K runs in the same order in every tile, so the tile changes no
+// result.  Operands in either layout save the transposed copies of weights,
+// activations and gradients.
+template <int EPI, bool TA, bool TB, int BM, int BN>
+__global__ void __launch_bounds__(128) k_gemm(const bf16 *__restrict__ A, int lda, const bf16 *__restrict__ B, int ldb,
+                                              int M, int N, int K, Epi epi) {
+    constexpr int ACH = TA ? BM / 8 : GK / 8, BCH = TB ? BN / 8 : GK / 8;  // chunks of a row
+    constexpr int AR = TA ? GK : BM, BR = TB ? GK : BN;                    // rows
+    constexpr int MI = BM / 32, NI = BN / 16;                              // m16 and n8 tiles of a warp
+    extern __shared__ __align__(128) unsigned char gsm[];
+    grid_launch_next();
+    grid_wait();
+    const unsigned as = (unsigned)__cvta_generic_to_shared(gsm), bs = as + GSTAGES * BM * GK * 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = (warp >> 1) * (BM / 2), wn = (warp & 1) * (BN / 2);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float acc[MI][NI][4] = {};
     auto load = [&](int st, int k0) {
-        // 64 rows x 32 bf16 = 64 x 4 chunks of 16 bytes, per operand
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int c = tid + 128 * q, row = c >> 2, col = (c & 3) * 8;
-            cp16(&As[st][row][col], A + (size_t)(m0 + row) * lda + k0 + col);
-            cp16(&Bs[st][row][col], B + (size_t)(n0 + row) * ldb + k0 + col);
+        for (int q = tid; q < AR * ACH; q += 128) {
+            const int r = q / ACH, c = q % ACH;
+            const bf16 *g = TA ? A + (size_t)(k0 + r) * lda + m0 + c * 8 : A + (size_t)(m0 + r) * lda + k0 + c * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                             as + st * BM * GK * 2 + (r * ACH + swz<ACH>(r, c)) * 16),
+                         "l"(g));
         }
-        asm volatile("cp.async.commit_group;\n" ::);
+#pragma unroll
+        for (int q = tid; q < BR * BCH; q += 128) {
+            const int r = q / BCH, c = q % BCH;
+            const bf16 *g = TB ? B + (size_t)(k0 + r) * ldb + n0 + c * 8 : B + (size_t)(n0 + r) * ldb + k0 + c * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                             bs + st * BN * GK * 2 + (r * BCH + swz<BCH>(r, c)) * 16),
+                         "l"(g));
+        }
     };
     const int nk = K / GK;
-    load(0, 0);
+#pragma unroll
+    for (int q = 0; q < GSTAGES - 1; q++) {
+        if (q < nk) load(q, q * GK);
+        asm volatile("cp.async.commit_group;\n" ::);
+    }
     for (int kt = 0; kt < nk; kt++) {
-        const int st = kt & 1;
-        if (kt + 1 < nk) {
-            load(st ^ 1, (kt + 1) * GK);
-            asm volatile("cp.async.wait_group 1;\n" ::);
-        } else {
-            asm volatile("cp.async.wait_group 0;\n" ::);
-        }
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(GSTAGES - 2) : "memory");
+        // stage kt has landed for every thread, and stage kt - 1 is used up
         __syncthreads();
+        if (kt + GSTAGES - 1 < nk) load((kt + GSTAGES - 1) % GSTAGES, (kt + GSTAGES - 1) * GK);
+        asm volatile("cp.async.commit_group;\n" ::);
+        const unsigned at = as + (kt % GSTAGES) * BM * GK * 2, bt = bs + (kt % GSTAGES) * BN * GK * 2;
 #pragma unroll
         for (int kk = 0; kk < GK; kk += 16) {
-            unsigned a[2][4], b[4][2];
+            unsigned a[MI][4], b[NI / 2][4];
 #pragma unroll
-            for (int mi = 0; mi < 2; mi++) {
-                const int r = 32 * wm + 16 * mi + g;
-                a[mi][0] = *reinterpret_cast<const unsigned *>(&As[st][r][kk + 2 * t]);
-                a[mi][1] = *reinterpret_cast<const unsigned *>(&As[st][r + 8][kk + 2 * t]);
-                a[mi][2] = *reinterpret_cast<const unsigned *>(&As[st][r][kk + 2 * t + 8]);
-                a[mi][3] = *reinterpret_cast<const unsigned *>(&As[st][r + 8][kk + 2 * t + 8]);
+            for (int mi = 0; mi < MI; mi++) {
+                const int mr = wm + 16 * mi;
+                const int r = TA ? kk + (lane & 7) + ((lane >> 4) << 3) : mr + (lane & 15);
+                const int c = TA ? mr / 8 + ((lane >> 3) & 1) : kk / 8 + (lane >> 4);
+                ldsm4<TA>(a[mi], at + (r * ACH + swz<ACH>(r, c)) * 16);
             }
 #pragma unroll
-            for (int ni = 0; ni < 4; ni++) {
-                const int c = 32 * wn + 8 * ni + g;
-                b[ni][0] = *reinterpret_cast<const unsigned *>(&Bs[st][c][kk + 2 * t]);
-                b[ni][1] = *reinterpret_cast<const unsigned *>(&Bs[st][c][kk + 2 * t + 8]);
+            for (int nj = 0; nj < NI / 2; nj++) {
+                const int nr = wn + 16 * nj;
+                const int r = TB ? kk + (lane & 15) : nr + (lane & 7) + ((lane >> 4) << 3);
+                const int c = TB ? nr / 8 + (lane >> 4) : kk / 8 + ((lane >> 3) & 1);
+                ldsm4<TB>(b[nj], bt + (r * BCH + swz<BCH>(r, c)) * 16);
             }
 #pragma unroll
-            for (int mi = 0; mi < 2; mi++)
+            for (int mi = 0; mi < MI; mi++)
 #pragma unroll
-                for (int ni = 0; ni < 4; ni++)
-                    mma_bf16(acc[mi][ni], a[mi][0], a[mi][1], a[mi][2], a[mi][3], b[ni][0], b[ni][1]);
+                for (int ni = 0; ni < NI; ni++)
+                    mma_bf16(acc[mi][ni], a[mi][0], a[mi][1], a[mi][2], a[mi][3], b[ni / 2][2 * (ni & 1)],
+                             b[ni / 2][2 * (ni & 1) + 1]);
         }
-        __syncthreads();  // the stage may be refilled
     }
     // epilogue: acc[mi][ni] covers rows r, r+8 and columns c, c+1
+    const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int mi = 0; mi < 2; mi++)
+    for (int mi = 0; mi < MI; mi++)
 #pragma unroll
-        for (int ni = 0; ni < 4; ni++)
+        for (int ni = 0; ni < NI; ni++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                const int r = m0 + 32 * wm + 16 * mi + g + 8 * h;
-                const int c = n0 + 32 * wn + 8 * ni + 2 * t;
+                const int r = m0 + wm + 16 * mi + g + 8 * h;
+                const int c = n0 + wn + 8 * ni + 2 * t;
                 float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
                 const size_t o = (size_t)r * N + c;
                 if (EPI == EPI_HIDDEN || EPI == EPI_OUT) {
                     v0 += epi.bias[c];
                     v1 += epi.bias[c + 1];
-                    epi.f32[o] = v0;
-                    epi.f32[o + 1] = v1;
+                    if (EPI == EPI_OUT || epi.f32) *reinterpret_cast<float2 *>(epi.f32 + o) = make_float2(v0, v1);
                     if (EPI == EPI_HIDDEN) {
                         __nv_bfloat162 p;
                         p.x = __float2bfloat16_rn(gelu(v0));
@@ -157,16 +208,17 @@ __global__ void __launch_bounds__(128) k_gemm_nt(const bf16 *__restrict__ A, int
                 } else if (EPI == EPI_BWD_GELU) {
                     v0 *= gelu_grad(epi.pre[o]);
                     v1 *= gelu_grad(epi.pre[o + 1]);
-                    epi.f32[o] = v0;
-                    epi.f32[o + 1] = v1;
-                    const bf16 b0 = __float2bfloat16_rn(v0), b1 = __float2bfloat16_rn(v1);
-                    epi.b16[o] = b0;
-                    epi.b16[o + 1] = b1;
-                    epi.b16t[(size_t)c * M + r] = b0;
-                    epi.b16t[(size_t)(c + 1) * M + r] = b1;
+                    *reinterpret_cast<float2 *>(epi.f32 + o) = make_float2(v0, v1);
+                    __nv_bfloat162 p;
+                    p.x = __float2bfloat16_rn(v0);
+                    p.y = __float2bfloat16_rn(v1);
+                    *reinterpret_cast<__nv_bfloat162 *>(epi.b16 + o) = p;
+                    if (epi.b16t) {
+                        epi.b16t[(size_t)c * M + r] = p.x;
+                        epi.b16t[(size_t)(c + 1) * M + r] = p.y;
+                    }
                 } else {
-                    epi.f32[o] = v0;
-                    epi.f32[o + 1] = v1;
+                    *reinterpret_cast<float2 *>(epi.f32 + o) = make_float2(v0, v1);
                 }
             }
 }
@@ -182,14 +234,14 @@ __global__ void __launch_bounds__(128) k_gemm_nt(const bf16 *__restrict__ A, int
 // stage for a later load; the last commit releases the accumulator, which
 // eight warps read back (tcgen05.ld, warp w lanes 32 (w % 4) .. +31 = tile
 // rows, columns 16 (w / 4) .. +15) into the same fused epilogues as
-// k_gemm_nt.  Every wait is bounded: on a timeout the CTA records it,
+// k_gemm.  Every wait is bounded: on a timeout the CTA records it,
 // waits (bounded) for its MMAs in flight, frees its tensor memory and
 // returns.  Measured on the surrogate's network (54-512x4-512, one B200):
-// a training step takes 0.226-0.233 ms at batch 256 against 0.189-0.191
-// ms on k_gemm_nt, and 0.51 against 0.42 ms at batch 2048 -- products of
-// at most 512 x 2048 x 512 are latency-bound on staging their tiles, which
-// this cp.async-fed form does no faster than the mma.sync tiles -- so it
-// runs only when asked for (RFSYN_FDTD_MLP_GEMM=tcgen05).
+// a training step takes 0.182 ms at batch 256 against 0.068 ms on k_gemm, and
+// 0.38 against 0.17 ms at batch 2048 -- products of at most 512 x 2048 x 512
+// are latency-bound on staging their tiles, which this cp.async-fed form does
+// no faster, and its operands need transposed copies -- so it runs only when
+// asked for (RFSYN_FDTD_MLP_GEMM=tcgen05).
 namespace tc {
 // Tiles of 128 rows x BN columns (BN 32: more CTAs on these small products
 // -- 128 x 128 tiles, fewer CTAs and fewer re-reads of A, measured slower
@@ -245,7 +297,7 @@ __device__ __forceinline__ void epi_store(const Epi &epi, int M, int N, int r, i
     const size_t o = (size_t)r * N + c;
     if (EPI == EPI_HIDDEN || EPI == EPI_OUT) {
         v += epi.bias[c];
-        epi.f32[o] = v;
+        if (EPI == EPI_OUT || epi.f32) epi.f32[o] = v;
         if (EPI == EPI_HIDDEN) epi.b16[o] = __float2bfloat16_rn(gelu(v));
     } else if (EPI == EPI_BWD_GELU) {
         v *= gelu_grad(epi.pre[o]);
@@ -381,6 +433,8 @@ __global__ void __launch_bounds__(tc::THREADS) k_gemm_tc(const bf16 *__restrict_
 __global__ void k_mse(const float *out, const float *y, int M, int N, float *d32, bf16 *d16, bf16 *d16t,
                       float *partial) {
     __shared__ float red[256];
+    grid_launch_next();
+    grid_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float se = 0.f;
     if (i < M * N) {
@@ -390,8 +444,10 @@ __global__ void k_mse(const float *out, const float *y, int M, int N, float *d32
         d32[i] = gr;
         const bf16 b = __float2bfloat16_rn(gr);
         d16[i] = b;
-        const int r = i / N, c = i - r * N;
-        d16t[(size_t)c * M + r] = b;
+        if (d16t) {
+            const int r = i / N, c = i - r * N;
+            d16t[(size_t)c * M + r] = b;
+        }
     }
     red[threadIdx.x] = se;
     __syncthreads();
@@ -421,52 +477,93 @@ __global__ void __launch_bounds__(256) k_colsum(const float *d, int M, int N, fl
     }
 }
 
-struct AdamArgs {
+// One parameter array (a layer's weights or its bias).
+struct AdamSeg {
     float *w, *m, *v;
     const float *g;
-    bf16 *w16, *w16t;    // weights as [rows][cols] and [cols][rows] BF16 (null for biases)
+    bf16 *w16, *w16t;    // BF16 copies [rows][cols] (null for biases) and [cols][rows] (or null)
     int n, rows, cols;
+};
+struct AdamCfg {
     float lr0, beta1, beta2, eps;
     long long total_steps;
-    const long long *step;  // steps done before this update
 };
 
-// Adam with bias correction; learning rate lr0 * 0.5 (1 + cos(pi s / S)).
-__global__ void k_adam(AdamArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const long long s = *a.step + 1;
-    const float frac = (float)min(1.0, (double)(s - 1) / (double)max(1LL, a.total_steps));
-    const float lr = a.lr0 * 0.5f * (1.0f + cospif(frac));
-    const float g = a.g[i];
-    const float m = a.beta1 * a.m[i] + (1.0f - a.beta1) * g;
-    const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * g * g;
-    a.m[i] = m;
-    a.v[i] = v;
-    const float mh = m / (1.0f - powf(a.beta1, (float)s));
-    const float vh = v / (1.0f - powf(a.beta2, (float)s));
-    const float w = a.w[i] - lr * mh / (sqrtf(vh) + a.eps);
-    a.w[i] = w;
-    if (a.w16) {
-        const bf16 b = __float2bfloat16_rn(w);
-        a.w16[i] = b;
-        const int r = i / a.cols, c = i - r * a.cols;
-        a.w16t[(size_t)c * a.rows + r] = b;
+constexpr int ADAM_BLOCK = 1024;  // parameters of a block, four a thread
+
+// Adam with bias correction over every parameter, learning rate lr0 * 0.5 (1
+// + cos(pi s / S)); block b takes the parameters from blocks[b].y on of
+// segs[blocks[b].x].  24 bytes a parameter move (and 2 of BF16), so one
+// launch of 16-byte accesses takes the place of one per array with scalar
+// ones: ten launches of 4.2-8.2 us, cold, for the 5-layer network, and two
+// powf a parameter, before.  The last block to finish advances *step (steps
+// done before this update), which every block has read by then.
+__global__ void __launch_bounds__(256) k_adam(const AdamSeg *segs, const int2 *blocks, const AdamCfg *cfg, long long *step,
+                                              int *done) {
+    __shared__ float s_lr, s_c1, s_c2;
+    grid_launch_next();
+    grid_wait();
+    const AdamCfg a = *cfg;
+    if (threadIdx.x == 0) {
+        const long long s = *step + 1;
+        const float frac = (float)min(1.0, (double)(s - 1) / (double)max(1LL, a.total_steps));
+        s_lr = a.lr0 * 0.5f * (1.0f + cospif(frac));
+        s_c1 = 1.0f - powf(a.beta1, (float)s);
+        s_c2 = 1.0f - powf(a.beta2, (float)s);
+    }
+    __syncthreads();
+    const float lr = s_lr, c1 = s_c1, c2 = s_c2;
+    const int2 b = blocks[blockIdx.x];
+    const AdamSeg sg = segs[b.x];
+    const int i = b.y + 4 * threadIdx.x;
+    if (i < sg.n) {
+        const float4 g4 = *reinterpret_cast<const float4 *>(sg.g + i);
+        float4 m4 = *reinterpret_cast<float4 *>(sg.m + i), v4 = *reinterpret_cast<float4 *>(sg.v + i),
+               w4 = *reinterpret_cast<float4 *>(sg.w + i);
+        const float *g = &g4.x;
+        float *m = &m4.x, *v = &v4.x, *w = &w4.x;
+        bf16 h[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            // the contractions nvcc chose for b m + (1 - b) g, written out so
+            // that the update stays the same bit for bit
+            m[q] = __fmaf_rn(1.0f - a.beta1, g[q], __fmul_rn(a.beta1, m[q]));
+            v[q] = __fmaf_rn(__fmul_rn(1.0f - a.beta2, g[q]), g[q], __fmul_rn(a.beta2, v[q]));
+            const float mh = m[q] / c1, vh = v[q] / c2;
+            w[q] = w[q] - lr * mh / (sqrtf(vh) + a.eps);
+            h[q] = __float2bfloat16_rn(w[q]);
+        }
+        *reinterpret_cast<float4 *>(sg.m + i) = m4;
+        *reinterpret_cast<float4 *>(sg.v + i) = v4;
+        *reinterpret_cast<float4 *>(sg.w + i) = w4;
+        if (sg.w16) *reinterpret_cast<uint2 *>(sg.w16 + i) = *reinterpret_cast<const uint2 *>(h);
+        if (sg.w16t) {
+            const int r = i / sg.cols, c = i - r * sg.cols;  // four columns of one row (cols a multiple of 4)
+#pragma unroll
+            for (int q = 0; q < 4; q++) sg.w16t[(size_t)(c + q) * sg.rows + r] = h[q];
+        }
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
+            *done = 0;
+            *step += 1;
+        }
     }
 }
-
-__global__ void k_step_inc(long long *step) { *step += 1; }
 
 // Batch of B rows from the resident set: row q of the batch is sample
 // perm[(step * B + q) mod n]; X as BF16 [B][kin] and its transpose, Y FP32.
 __global__ void k_gather(const bf16 *X, const float *Y, const int *perm, long long n, const long long *step, int B,
                          int kin, int nout, bf16 *xb, bf16 *xbt, float *yb) {
+    grid_launch_next();
     const int q = blockIdx.x;
+    grid_wait();
     const long long idx = perm[((*step) * B + q) % n];
     for (int c = threadIdx.x; c < kin; c += blockDim.x) {
         const bf16 v = X[idx * kin + c];
         xb[(size_t)q * kin + c] = v;
-        xbt[(size_t)c * B + q] = v;
+        if (xbt) xbt[(size_t)c * B + q] = v;
     }
     for (int c = threadIdx.x; c < nout; c += blockDim.x) yb[(size_t)q * nout + c] = Y[idx * nout + c];
 }
@@ -505,20 +602,31 @@ struct fdtd_b200_mlp {
     int bmax = 0;                          // batch buffers sized for this many rows
     std::vector<float *> pre;              // per hidden layer [B][width]
     std::vector<bf16 *> act, actt;         // per layer input: act[0] = x, act[l] = GELU(pre[l-1]); transposes
-    float *out = nullptr, *y = nullptr, *d32 = nullptr, *partial = nullptr;
-    bf16 *d16 = nullptr, *d16t = nullptr;
-    float *dz32 = nullptr;
-    bf16 *dz16 = nullptr, *dz16t = nullptr;
+    float *out = nullptr, *y = nullptr, *partial = nullptr;
+    // gradient at each layer's output, FP32 and BF16 (and transposed for the
+    // tcgen05 products): one set a layer, as the weight gradients of a layer
+    // run while the next ones are computed
+    std::vector<float *> g32;
+    std::vector<bf16 *> g16, g16t;
+    float *xf = nullptr;                   // bmax FP32 input rows on their way to BF16
+    void *batch_mem = nullptr, *param_mem = nullptr;  // the blocks of the batch and of the parameter arrays
     // resident training set
     bf16 *X = nullptr;
     float *Y = nullptr;
     int *perm = nullptr;
     size_t n_data = 0;
     long long *step = nullptr;
-    cudaStream_t st = nullptr;
-    cudaGraphExec_t graph = nullptr;
+    cudaStream_t st = nullptr, st_w = nullptr, st_b = nullptr;  // main; weight and bias gradients
+    std::vector<cudaEvent_t> ev_g;         // gradient of layer l ready
+    cudaEvent_t ev_w = nullptr, ev_b = nullptr;
+    // training graphs of one step and of GRAPH_STEPS, for batches of graph_b
+    cudaGraphExec_t graph = nullptr, graph_n = nullptr;
     int graph_b = 0;
-    AdamArgs adam_cfg{};
+    AdamCfg *cfg = nullptr;
+    bool overlap = false;                  // launches are being captured as programmatic dependents
+    AdamSeg *segs = nullptr;
+    int2 *blocks = nullptr;
+    int n_blocks = 0, *done = nullptr;
     unsigned long long launches = 0;
     // tensor-core products: enabled (the shared memory attribute was set),
     // their launches, and the device flag a timed-out wait sets
@@ -538,67 +646,111 @@ typedef struct fdtd_b200_mlp fdtd_b200_mlp_t;
         }                                                                                     \
     } while (0)
 
+// Sub-arrays of one block, on 256-byte boundaries: a driver allocation costs
+// up to milliseconds, whatever its size.
+struct Arena {
+    char *base;
+    size_t used = 0;
+    template <typename X>
+    void take(X *&p, size_t n) {
+        p = base ? reinterpret_cast<X *>(base + used) : nullptr;
+        used += (n * sizeof(X) + 255) / 256 * 256;
+    }
+};
+
+static void mlp_free_graphs(fdtd_b200_mlp *m) {
+    for (cudaGraphExec_t *g : {&m->graph, &m->graph_n}) {
+        if (*g) cudaGraphExecDestroy(*g);
+        *g = nullptr;
+    }
+}
+
 static void mlp_free_batch(fdtd_b200_mlp *m) {
-    for (auto p : m->pre) cudaFree(p);
-    for (auto p : m->act) cudaFree(p);
-    for (auto p : m->actt) cudaFree(p);
-    m->pre.clear();
-    m->act.clear();
-    m->actt.clear();
-    cudaFree(m->out); cudaFree(m->y); cudaFree(m->d32); cudaFree(m->partial);
-    cudaFree(m->d16); cudaFree(m->d16t); cudaFree(m->dz32); cudaFree(m->dz16); cudaFree(m->dz16t);
-    m->out = m->y = m->d32 = m->partial = m->dz32 = nullptr;
-    m->d16 = m->d16t = m->dz16 = m->dz16t = nullptr;
-    if (m->graph) cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
+    cudaFree(m->batch_mem);
+    m->batch_mem = nullptr;
+    mlp_free_graphs(m);
     m->bmax = 0;
+}
+
+static size_t mlp_lay_batch(fdtd_b200_mlp *m, int B, char *base) {
+    const int nl = (int)m->L.size();
+    Arena a{base};
+    m->pre.assign(nl - 1, nullptr);
+    m->act.assign(nl, nullptr);
+    m->actt.assign(nl, nullptr);
+    m->g32.assign(nl, nullptr);
+    m->g16.assign(nl, nullptr);
+    m->g16t.assign(nl, nullptr);
+    for (int l = 0; l < nl; l++) {
+        const size_t ni = (size_t)B * m->L[l].in, no = (size_t)B * m->L[l].out;
+        a.take(m->act[l], ni);
+        a.take(m->g32[l], no);
+        a.take(m->g16[l], no);
+        if (m->tc) {
+            a.take(m->actt[l], ni);
+            a.take(m->g16t[l], no);
+        }
+        if (l < nl - 1) a.take(m->pre[l], no);
+    }
+    const size_t no = (size_t)B * m->n_out;
+    a.take(m->out, no);
+    a.take(m->y, no);
+    a.take(m->partial, no / 256 + 1);
+    a.take(m->xf, (size_t)B * m->n_in);
+    return a.used;
 }
 
 static int mlp_batch_buffers(fdtd_b200_mlp *m, int B) {
     if (B <= m->bmax) return 0;
     mlp_free_batch(m);
-    const int nl = (int)m->L.size();
-    m->pre.assign(nl - 1, nullptr);
-    m->act.assign(nl, nullptr);
-    m->actt.assign(nl, nullptr);
-    for (int l = 0; l < nl; l++) {
-        MCK(cudaMalloc(&m->act[l], (size_t)B * m->L[l].in * sizeof(bf16)));
-        MCK(cudaMalloc(&m->actt[l], (size_t)B * m->L[l].in * sizeof(bf16)));
-        if (l < nl - 1) MCK(cudaMalloc(&m->pre[l], (size_t)B * m->L[l].out * sizeof(float)));
-    }
-    // the two gradient buffer sets alternate between output-sized and
-    // hidden-sized gradients: both hold the larger
-    const size_t no = (size_t)B * m->n_out, nw = (size_t)B * std::max(m->width, m->n_out);
-    MCK(cudaMalloc(&m->out, no * sizeof(float)));
-    MCK(cudaMalloc(&m->y, no * sizeof(float)));
-    MCK(cudaMalloc(&m->d32, nw * sizeof(float)));
-    MCK(cudaMalloc(&m->d16, nw * sizeof(bf16)));
-    MCK(cudaMalloc(&m->d16t, nw * sizeof(bf16)));
-    MCK(cudaMalloc(&m->partial, (no / 256 + 1) * sizeof(float)));
-    MCK(cudaMalloc(&m->dz32, nw * sizeof(float)));
-    MCK(cudaMalloc(&m->dz16, nw * sizeof(bf16)));
-    MCK(cudaMalloc(&m->dz16t, nw * sizeof(bf16)));
+    MCK(cudaMalloc(&m->batch_mem, mlp_lay_batch(m, B, nullptr)));
+    mlp_lay_batch(m, B, static_cast<char *>(m->batch_mem));
     m->bmax = B;
     return 0;
 }
 
-// The network's products: k_gemm_nt (64 x 64 tiles, mma.sync), or with
-// RFSYN_FDTD_MLP_GEMM=tcgen05 k_gemm_tc where the shapes fit its tiles (M a
+// The network's products on k_gemm, or with RFSYN_FDTD_MLP_GEMM=tcgen05 on
+// k_gemm_tc where both operands are K-major and the shapes fit its tiles (M a
 // multiple of 128, N of 32, K of 64 -- every training-step product of the
-// surrogate does).
-template <int EPI>
-static void gemm(fdtd_b200_mlp *m, const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N, int K, Epi epi) {
-    if (m->tc && M > 0 && N > 0 && K > 0 && M % tc::BM == 0 && N % 32 == 0 && K % tc::BK == 0 && lda % 8 == 0 &&
-        ldb % 8 == 0) {
-        dim3 grid(N / 32, M / tc::BM);
-        k_gemm_tc<EPI, 32><<<grid, tc::THREADS, tc::Shape<32>::SMEM, m->st>>>(A, lda, B, ldb, M, N, K, epi,
-                                                                            m->d_err);
-        m->tc_launches++;
-    } else {
-        dim3 grid(N / GT, M / GT);
-        k_gemm_nt<EPI><<<grid, 128, 0, m->st>>>(A, lda, B, ldb, M, N, K, epi);
+// surrogate does).  64 x 64 tiles once they give every SM a CTA: half the
+// operand re-reads of 32 x 32 tiles, which a smaller product needs for CTAs
+// (256 x 512 outputs: 32 against 128).
+template <int BM>
+constexpr int gemm_smem() {
+    return GSTAGES * 2 * BM * GK * (int)sizeof(bf16);
+}
+template <int EPI, bool TA = false, bool TB = false>
+static void gemm(fdtd_b200_mlp *m, cudaStream_t st, const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N, int K,
+                 Epi epi) {
+    if constexpr (!TA && !TB) {
+        if (m->tc && M > 0 && N > 0 && K > 0 && M % tc::BM == 0 && N % 32 == 0 && K % tc::BK == 0 && lda % 8 == 0 &&
+            ldb % 8 == 0) {
+            dim3 grid(N / 32, M / tc::BM);
+            k_gemm_tc<EPI, 32><<<grid, tc::THREADS, tc::Shape<32>::SMEM, st>>>(A, lda, B, ldb, M, N, K, epi, m->d_err);
+            m->tc_launches++;
+            m->launches++;
+            return;
+        }
     }
+    // the products of the main stream's chain are programmatic dependents
+    const bool overlap = m->overlap && st == m->st;
+    if ((long long)(M / 64) * (N / 64) >= 148)
+        launch_step(k_gemm<EPI, TA, TB, 64, 64>, dim3(N / 64, M / 64), dim3(128), gemm_smem<64>(), st, overlap, A, lda, B,
+                    ldb, M, N, K, epi);
+    else
+        launch_step(k_gemm<EPI, TA, TB, 32, 32>, dim3(N / 32, M / 32), dim3(128), gemm_smem<32>(), st, overlap, A, lda, B,
+                    ldb, M, N, K, epi);
     m->launches++;
+}
+template <int EPI, bool TA, bool TB>
+static bool gemm_attr() {
+    return cudaFuncSetAttribute(k_gemm<EPI, TA, TB, 64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                gemm_smem<64>()) == cudaSuccess;
+}
+static bool gemm_attrs() {
+    return gemm_attr<EPI_HIDDEN, false, false>() && gemm_attr<EPI_OUT, false, false>() &&
+           gemm_attr<EPI_BWD_GELU, false, false>() && gemm_attr<EPI_BWD_GELU, false, true>() &&
+           gemm_attr<EPI_F32, false, false>() && gemm_attr<EPI_F32, true, true>();
 }
 
 // The tensor-core products need more than 48 KB of shared memory.
@@ -630,26 +782,27 @@ static int mlp_check_err(fdtd_b200_mlp *m) {
     return 0;
 }
 
-// Forward pass of B rows whose input is already in act[0].
-static void mlp_forward(fdtd_b200_mlp *m, int B) {
+// Forward pass of B rows whose input is already in act[0]; the hidden
+// pre-activations are kept when a backward pass follows.
+static void mlp_forward(fdtd_b200_mlp *m, int B, bool keep) {
     const int nl = (int)m->L.size();
     for (int l = 0; l < nl; l++) {
         const Layer &ly = m->L[l];
         Epi e{};
         e.bias = ly.b;
         if (l < nl - 1) {
-            e.f32 = m->pre[l];
+            e.f32 = keep ? m->pre[l] : nullptr;
             e.b16 = m->act[l + 1];
-            gemm<EPI_HIDDEN>(m, m->act[l], ly.in, ly.w16, ly.in, B, ly.out, ly.in, e);
+            gemm<EPI_HIDDEN>(m, m->st, m->act[l], ly.in, ly.w16, ly.in, B, ly.out, ly.in, e);
         } else {
             e.f32 = m->out;
-            gemm<EPI_OUT>(m, m->act[l], ly.in, ly.w16, ly.in, B, ly.out, ly.in, e);
+            gemm<EPI_OUT>(m, m->st, m->act[l], ly.in, ly.w16, ly.in, B, ly.out, ly.in, e);
         }
     }
 }
 
 // Transposes of the hidden activations (B x width, BF16) for the weight
-// gradients: written by a small kernel.
+// gradients on the tcgen05 products: written by a small kernel.
 __global__ void k_transpose_bf16(const bf16 *in, int rows, int cols, bf16 *out) {
     __shared__ bf16 tile[32][33];
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -660,64 +813,82 @@ __global__ void k_transpose_bf16(const bf16 *in, int rows, int cols, bf16 *out) 
         if (c0 + y < cols && r0 + threadIdx.x < rows) out[(size_t)(c0 + y) * rows + r0 + threadIdx.x] = tile[threadIdx.x][y];
 }
 
-// Backward pass after the forward (dOut already in d32 / d16 / d16t): weight
-// and bias gradients of every layer.  The gradient flowing backwards
-// alternates between the (d*) and (dz*) buffer sets.
-static void mlp_backward(fdtd_b200_mlp *m, int B) {
+// Backward pass after the forward (the output gradient already in the last
+// layer's buffers): weight and bias gradients of every layer.  The chain of
+// dX products runs on the main stream; each layer's weight gradient and bias
+// sums follow on two streams of their own as its gradient is ready, and the
+// main stream waits for both at the end.
+static int mlp_backward(fdtd_b200_mlp *m, int B) {
     const int nl = (int)m->L.size();
-    // transposes of the layer inputs (act[0]^T is written by the gather)
-    for (int l = 1; l < nl; l++) {
-        dim3 grid((m->L[l].in + 31) / 32, (B + 31) / 32);
-        k_transpose_bf16<<<grid, dim3(32, 8), 0, m->st>>>(m->act[l], B, m->L[l].in, m->actt[l]);
-        m->launches++;
-    }
-    float *g32[2] = {m->d32, m->dz32};
-    bf16 *g16[2] = {m->d16, m->dz16}, *g16t[2] = {m->d16t, m->dz16t};
-    int cur = 0;
+    if (m->tc)
+        // transposes of the layer inputs (act[0]^T is written by the gather)
+        for (int l = 1; l < nl; l++) {
+            dim3 grid((m->L[l].in + 31) / 32, (B + 31) / 32);
+            k_transpose_bf16<<<grid, dim3(32, 8), 0, m->st>>>(m->act[l], B, m->L[l].in, m->actt[l]);
+            m->launches++;
+        }
     for (int l = nl - 1; l >= 0; l--) {
         const Layer &ly = m->L[l];
-        // dW = dZ^T . X: [out][in] = (dZ^T [out][B]) . (X^T [in][B])^T
+        MCK(cudaEventRecord(m->ev_g[l], m->st));
+        MCK(cudaStreamWaitEvent(m->st_w, m->ev_g[l], 0));
+        MCK(cudaStreamWaitEvent(m->st_b, m->ev_g[l], 0));
+        // dW = dZ^T . X: [out][in] from dZ [B][out] and X [B][in]
         Epi e{};
         e.f32 = ly.gw;
-        gemm<EPI_F32>(m, g16t[cur], B, m->actt[l], B, ly.out, ly.in, B, e);
-        k_colsum<<<(ly.out + 31) / 32, 256, 0, m->st>>>(g32[cur], B, ly.out, ly.gb);
+        if (m->tc) gemm<EPI_F32>(m, m->st_w, m->g16t[l], B, m->actt[l], B, ly.out, ly.in, B, e);
+        else gemm<EPI_F32, true, true>(m, m->st_w, m->g16[l], ly.out, m->act[l], ly.in, ly.out, ly.in, B, e);
+        k_colsum<<<(ly.out + 31) / 32, 256, 0, m->st_b>>>(m->g32[l], B, ly.out, ly.gb);
         m->launches++;
         if (l > 0) {
-            // dX = dZ . W = dZ [B][out] . (W^T [in][out])^T, times GELU' of the
-            // previous layer's pre-activation
+            // dX = dZ . W, W [out][in], times GELU' of the previous layer's
+            // pre-activation
             Epi eb{};
-            eb.f32 = g32[cur ^ 1];
-            eb.b16 = g16[cur ^ 1];
-            eb.b16t = g16t[cur ^ 1];
+            eb.f32 = m->g32[l - 1];
+            eb.b16 = m->g16[l - 1];
+            eb.b16t = m->g16t[l - 1];
             eb.pre = m->pre[l - 1];
-            gemm<EPI_BWD_GELU>(m, g16[cur], ly.out, ly.w16t, ly.out, B, ly.in, ly.out, eb);
-            cur ^= 1;
+            if (m->tc) gemm<EPI_BWD_GELU>(m, m->st, m->g16[l], ly.out, ly.w16t, ly.out, B, ly.in, ly.out, eb);
+            else gemm<EPI_BWD_GELU, false, true>(m, m->st, m->g16[l], ly.out, ly.w16, ly.in, B, ly.in, ly.out, eb);
         }
     }
+    MCK(cudaEventRecord(m->ev_w, m->st_w));
+    MCK(cudaEventRecord(m->ev_b, m->st_b));
+    MCK(cudaStreamWaitEvent(m->st, m->ev_w, 0));
+    MCK(cudaStreamWaitEvent(m->st, m->ev_b, 0));
+    return 0;
 }
 
 static void mlp_loss(fdtd_b200_mlp *m, int B) {
     const int n = B * m->n_out;
-    k_mse<<<(n + 255) / 256, 256, 0, m->st>>>(m->out, m->y, B, m->n_out, m->d32, m->d16, m->d16t, m->partial);
+    launch_step(k_mse, dim3((n + 255) / 256), dim3(256), 0, m->st, m->overlap, m->out, m->y, B, m->n_out, m->g32.back(),
+                m->g16.back(), m->g16t.back(), m->partial);
     m->launches++;
 }
 
 static void mlp_adam(fdtd_b200_mlp *m) {
-    for (Layer &ly : m->L) {
-        AdamArgs a = m->adam_cfg;
-        a.w = ly.w; a.m = ly.mw; a.v = ly.vw; a.g = ly.gw;
-        a.w16 = ly.w16; a.w16t = ly.w16t;
-        a.n = ly.out * ly.in; a.rows = ly.out; a.cols = ly.in;
-        k_adam<<<(a.n + 255) / 256, 256, 0, m->st>>>(a);
-        AdamArgs b = m->adam_cfg;
-        b.w = ly.b; b.m = ly.mb; b.v = ly.vb; b.g = ly.gb;
-        b.w16 = nullptr; b.w16t = nullptr;
-        b.n = ly.out; b.rows = 1; b.cols = ly.out;
-        k_adam<<<(b.n + 255) / 256, 256, 0, m->st>>>(b);
-        m->launches += 2;
-    }
-    k_step_inc<<<1, 1, 0, m->st>>>(m->step);
+    k_adam<<<m->n_blocks, 256, 0, m->st>>>(m->segs, m->blocks, m->cfg, m->step, m->done);
     m->launches++;
+}
+
+// The parameter arrays and blocks of k_adam.
+static int mlp_adam_segs(fdtd_b200_mlp *m) {
+    std::vector<AdamSeg> segs;
+    std::vector<int2> blocks;
+    for (Layer &ly : m->L) {
+        segs.push_back(AdamSeg{ly.w, ly.mw, ly.vw, ly.gw, ly.w16, ly.w16t, ly.out * ly.in, ly.out, ly.in});
+        segs.push_back(AdamSeg{ly.b, ly.mb, ly.vb, ly.gb, nullptr, nullptr, ly.out, 1, ly.out});
+    }
+    for (size_t q = 0; q < segs.size(); q++)
+        for (int o = 0; o < segs[q].n; o += ADAM_BLOCK) blocks.push_back(make_int2((int)q, o));
+    m->n_blocks = (int)blocks.size();
+    MCK(cudaMalloc(&m->segs, segs.size() * sizeof(AdamSeg)));
+    MCK(cudaMalloc(&m->blocks, blocks.size() * sizeof(int2)));
+    MCK(cudaMalloc(&m->done, sizeof(int)));
+    MCK(cudaMalloc(&m->cfg, sizeof(AdamCfg)));
+    MCK(cudaMemcpy(m->segs, segs.data(), segs.size() * sizeof(AdamSeg), cudaMemcpyHostToDevice));
+    MCK(cudaMemcpy(m->blocks, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    MCK(cudaMemset(m->done, 0, sizeof(int)));
+    return 0;
 }
 
 // BF16 copies (and transposes) of the FP32 master weights.
@@ -725,9 +896,11 @@ static int mlp_sync_bf16(fdtd_b200_mlp *m) {
     for (Layer &ly : m->L) {
         const size_t n = (size_t)ly.out * ly.in;
         k_f2bf<<<(unsigned)((n + 255) / 256), 256, 0, m->st>>>(ly.w, ly.w16, n);
+        m->launches++;
+        if (!m->tc) continue;
         dim3 grid((ly.in + 31) / 32, (ly.out + 31) / 32);
         k_transpose_bf16<<<grid, dim3(32, 8), 0, m->st>>>(ly.w16, ly.out, ly.in, ly.w16t);
-        m->launches += 2;
+        m->launches++;
     }
     MCK(cudaGetLastError());
     return 0;
@@ -737,12 +910,14 @@ extern "C" void fdtd_b200_mlp_destroy(fdtd_b200_mlp_t *m) {
     if (!m) return;
     if (m->st) cudaStreamSynchronize(m->st);
     mlp_free_batch(m);
-    for (Layer &ly : m->L) {
-        cudaFree(ly.w); cudaFree(ly.b); cudaFree(ly.mw); cudaFree(ly.vw); cudaFree(ly.mb); cudaFree(ly.vb);
-        cudaFree(ly.gw); cudaFree(ly.gb); cudaFree(ly.w16); cudaFree(ly.w16t);
-    }
+    cudaFree(m->param_mem);
     cudaFree(m->X); cudaFree(m->Y); cudaFree(m->perm); cudaFree(m->step); cudaFree(m->d_err);
-    if (m->st) cudaStreamDestroy(m->st);
+    cudaFree(m->segs); cudaFree(m->blocks); cudaFree(m->done); cudaFree(m->cfg);
+    for (cudaEvent_t ev : m->ev_g) cudaEventDestroy(ev);
+    if (m->ev_w) cudaEventDestroy(m->ev_w);
+    if (m->ev_b) cudaEventDestroy(m->ev_b);
+    for (cudaStream_t st : {m->st, m->st_w, m->st_b})
+        if (st) cudaStreamDestroy(st);
     delete m;
 }
 
@@ -776,42 +951,21 @@ extern "C" fdtd_b200_mlp_t *fdtd_b200_mlp_create(int n_in, int width, int depth,
         fdtd_b200_mlp_destroy(m);
         return nullptr;
     };
-    if (cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking) != cudaSuccess) return fail();
-    for (int l = 0; l <= depth; l++) {
-        Layer &ly = m->L[l];
-        const size_t nw = (size_t)ly.out * ly.in;
-        float **f32s[] = {&ly.w, &ly.mw, &ly.vw, &ly.gw};
-        for (float **p : f32s)
-            if (cudaMalloc(p, nw * sizeof(float)) != cudaSuccess) return fail();
-        float **b32s[] = {&ly.b, &ly.mb, &ly.vb, &ly.gb};
-        for (float **p : b32s)
-            if (cudaMalloc(p, ly.out * sizeof(float)) != cudaSuccess) return fail();
-        if (cudaMalloc(&ly.w16, nw * sizeof(bf16)) != cudaSuccess) return fail();
-        if (cudaMalloc(&ly.w16t, nw * sizeof(bf16)) != cudaSuccess) return fail();
-        // uniform(-lim, lim), lim = sqrt(6 / fan_in) (He); only the real inputs
-        // of the first layer count, padded columns start at zero
-        const int fan_in = l == 0 ? n_in : ly.in;
-        const double lim = sqrt(6.0 / fan_in) * (l == depth ? 0.5 : 1.0);
-        std::vector<float> w(nw, 0.f), z(nw, 0.f), zb(ly.out, 0.f);
-        for (int r = 0; r < ly.out; r++)
-            for (int c = 0; c < ly.in; c++) {
-                const double u = (double)(splitmix(rs) >> 11) * (1.0 / 9007199254740992.0);
-                w[(size_t)r * ly.in + c] = (l == 0 && c >= n_in) ? 0.f : (float)((2.0 * u - 1.0) * lim);
-            }
-        if (cudaMemcpy(ly.w, w.data(), nw * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
-        if (cudaMemcpy(ly.mw, z.data(), nw * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
-        if (cudaMemcpy(ly.vw, z.data(), nw * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
-        if (cudaMemcpy(ly.b, zb.data(), ly.out * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
-        if (cudaMemcpy(ly.mb, zb.data(), ly.out * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
-        if (cudaMemcpy(ly.vb, zb.data(), ly.out * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
+    for (cudaStream_t *st : {&m->st, &m->st_w, &m->st_b})
+        if (cudaStreamCreateWithFlags(st, cudaStreamNonBlocking) != cudaSuccess) return fail();
+    m->ev_g.assign(depth + 1, nullptr);
+    for (cudaEvent_t &ev : m->ev_g)
+        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return fail();
+    if (cudaEventCreateWithFlags(&m->ev_w, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&m->ev_b, cudaEventDisableTiming) != cudaSuccess)
+        return fail();
+    if (!gemm_attrs()) {
+        rfb_set_error("mlp: cannot configure the products' shared memory");
+        return fail();
     }
-    if (cudaMalloc(&m->step, sizeof(long long)) != cudaSuccess) return fail();
-    if (cudaMemset(m->step, 0, sizeof(long long)) != cudaSuccess) return fail();
-    if (cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) return fail();
-    if (cudaMemset(m->d_err, 0, sizeof(int)) != cudaSuccess) return fail();
     {
         // RFSYN_FDTD_MLP_GEMM=tcgen05 puts the products whose shapes fit on
-        // k_gemm_tc; by default every product runs on k_gemm_nt, which is
+        // k_gemm_tc; by default every product runs on k_gemm, which is
         // faster on this network's products at every batch measured (see
         // k_gemm_tc)
         const char *v = getenv("RFSYN_FDTD_MLP_GEMM");
@@ -822,6 +976,41 @@ extern "C" fdtd_b200_mlp_t *fdtd_b200_mlp_create(int n_in, int width, int depth,
             return fail();
         }
     }
+    auto lay = [&](char *base) {
+        Arena a{base};
+        for (Layer &ly : m->L) {
+            const size_t nw = (size_t)ly.out * ly.in;
+            for (float **p : {&ly.w, &ly.mw, &ly.vw, &ly.gw}) a.take(*p, nw);
+            for (float **p : {&ly.b, &ly.mb, &ly.vb, &ly.gb}) a.take(*p, (size_t)ly.out);
+            a.take(ly.w16, nw);
+            if (m->tc) a.take(ly.w16t, nw);
+        }
+        return a.used;
+    };
+    const size_t param_bytes = lay(nullptr);
+    if (cudaMalloc(&m->param_mem, param_bytes) != cudaSuccess) return fail();
+    if (cudaMemset(m->param_mem, 0, param_bytes) != cudaSuccess) return fail();
+    lay(static_cast<char *>(m->param_mem));
+    for (int l = 0; l <= depth; l++) {
+        Layer &ly = m->L[l];
+        const size_t nw = (size_t)ly.out * ly.in;
+        // uniform(-lim, lim), lim = sqrt(6 / fan_in) (He); only the real inputs
+        // of the first layer count, padded columns start at zero
+        const int fan_in = l == 0 ? n_in : ly.in;
+        const double lim = sqrt(6.0 / fan_in) * (l == depth ? 0.5 : 1.0);
+        std::vector<float> w(nw, 0.f);
+        for (int r = 0; r < ly.out; r++)
+            for (int c = 0; c < ly.in; c++) {
+                const double u = (double)(splitmix(rs) >> 11) * (1.0 / 9007199254740992.0);
+                w[(size_t)r * ly.in + c] = (l == 0 && c >= n_in) ? 0.f : (float)((2.0 * u - 1.0) * lim);
+            }
+        if (cudaMemcpy(ly.w, w.data(), nw * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail();
+    }
+    if (cudaMalloc(&m->step, sizeof(long long)) != cudaSuccess) return fail();
+    if (cudaMemset(m->step, 0, sizeof(long long)) != cudaSuccess) return fail();
+    if (cudaMalloc(&m->d_err, sizeof(int)) != cudaSuccess) return fail();
+    if (cudaMemset(m->d_err, 0, sizeof(int)) != cudaSuccess) return fail();
+    if (mlp_adam_segs(m) != 0) return fail();
     if (mlp_sync_bf16(m) != 0) return fail();
     if (cudaStreamSynchronize(m->st) != cudaSuccess) return fail();
     return m;
@@ -875,21 +1064,14 @@ static int mlp_read_grads(fdtd_b200_mlp *m, float *out) {
     return 0;
 }
 
-static int mlp_upload_x(fdtd_b200_mlp *m, const float *X, size_t n, bf16 *dst) {
-    float *tmp = nullptr;
-    MCK(cudaMalloc(&tmp, n * m->n_in * sizeof(float)));
-    cudaError_t e = cudaMemcpyAsync(tmp, X, n * m->n_in * sizeof(float), cudaMemcpyHostToDevice, m->st);
-    if (e == cudaSuccess) {
-        const size_t tot = n * m->kin;
-        k_pack_x<<<(unsigned)((tot + 255) / 256), 256, 0, m->st>>>(tmp, m->n_in, dst, m->kin, n);
-        m->launches++;
-        e = cudaStreamSynchronize(m->st);
-    }
-    cudaFree(tmp);
-    if (e != cudaSuccess) {
-        rfb_set_error("mlp: input upload failed: %s", cudaGetErrorString(e));
-        return -1;
-    }
+// n rows of host X as BF16 rows [n][kin] in dst through the FP32 rows xf
+// (queued on the main stream; X may be reused once the stream has passed).
+static int mlp_upload_x(fdtd_b200_mlp *m, const float *X, size_t n, bf16 *dst, float *xf) {
+    MCK(cudaMemcpyAsync(xf, X, n * m->n_in * sizeof(float), cudaMemcpyHostToDevice, m->st));
+    const size_t tot = n * m->kin;
+    k_pack_x<<<(unsigned)((tot + 255) / 256), 256, 0, m->st>>>(xf, m->n_in, dst, m->kin, n);
+    m->launches++;
+    MCK(cudaGetLastError());
     return 0;
 }
 
@@ -902,13 +1084,15 @@ extern "C" int fdtd_b200_mlp_grad(fdtd_b200_mlp_t *m, const float *X, const floa
         return -1;
     }
     if (mlp_batch_buffers(m, B) != 0) return -1;
-    if (mlp_upload_x(m, X, B, m->act[0]) != 0) return -1;
-    dim3 grid((m->kin + 31) / 32, (B + 31) / 32);
-    k_transpose_bf16<<<grid, dim3(32, 8), 0, m->st>>>(m->act[0], B, m->kin, m->actt[0]);
+    if (mlp_upload_x(m, X, B, m->act[0], m->xf) != 0) return -1;
+    if (m->tc) {
+        dim3 grid((m->kin + 31) / 32, (B + 31) / 32);
+        k_transpose_bf16<<<grid, dim3(32, 8), 0, m->st>>>(m->act[0], B, m->kin, m->actt[0]);
+    }
     MCK(cudaMemcpyAsync(m->y, Y, (size_t)B * m->n_out * 4, cudaMemcpyHostToDevice, m->st));
-    mlp_forward(m, B);
+    mlp_forward(m, B, true);
     mlp_loss(m, B);
-    mlp_backward(m, B);
+    if (mlp_backward(m, B) != 0) return -1;
     MCK(cudaGetLastError());
     std::vector<float> part((size_t)B * m->n_out / 256 + 1);
     const int nb = (B * m->n_out + 255) / 256;
@@ -934,22 +1118,52 @@ extern "C" int fdtd_b200_mlp_set_data(fdtd_b200_mlp_t *m, const float *X, const 
     MCK(cudaMalloc(&m->X, n * m->kin * sizeof(bf16)));
     MCK(cudaMalloc(&m->Y, n * m->n_out * sizeof(float)));
     MCK(cudaMalloc(&m->perm, n * sizeof(int)));
-    if (mlp_upload_x(m, X, n, m->X) != 0) return -1;
+    {
+        // the whole data set's staging is not kept
+        float *xf = nullptr;
+        MCK(cudaMalloc(&xf, n * m->n_in * sizeof(float)));
+        const int rc = mlp_upload_x(m, X, n, m->X, xf);
+        const cudaError_t e = cudaStreamSynchronize(m->st);
+        cudaFree(xf);
+        if (rc != 0) return -1;
+        MCK(e);
+    }
     MCK(cudaMemcpy(m->Y, Y, n * m->n_out * sizeof(float), cudaMemcpyHostToDevice));
     m->n_data = n;
-    if (m->graph) cudaGraphExecDestroy(m->graph);
-    m->graph = nullptr;
+    mlp_free_graphs(m);
     return 0;
 }
 
-static void mlp_train_step(fdtd_b200_mlp *m, int B) {
-    k_gather<<<B, 128, 0, m->st>>>(m->X, m->Y, m->perm, (long long)m->n_data, m->step, B, m->kin, m->n_out,
-                                   m->act[0], m->actt[0], m->y);
+static int mlp_train_step(fdtd_b200_mlp *m, int B, bool first) {
+    launch_step(k_gather, dim3(B), dim3(128), 0, m->st, m->overlap && !first, m->X, m->Y, m->perm, (long long)m->n_data,
+                m->step, B, m->kin, m->n_out, m->act[0], m->actt[0], m->y);
     m->launches++;
-    mlp_forward(m, B);
+    mlp_forward(m, B, true);
     mlp_loss(m, B);
-    mlp_backward(m, B);
+    if (mlp_backward(m, B) != 0) return -1;
     mlp_adam(m);
+    return 0;
+}
+
+// Captures `steps` training steps.  The graphs hold the batch buffers and the
+// data set, not the schedule (cfg, step), so they serve every later call.
+static int mlp_capture(fdtd_b200_mlp *m, int B, int steps, cudaGraphExec_t *out) {
+    cudaGraph_t g = nullptr;
+    MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
+    m->overlap = !m->tc;
+    int rc = 0;
+    for (int s = 0; s < steps && rc == 0; s++) rc = mlp_train_step(m, B, s == 0);
+    m->overlap = false;
+    const cudaError_t ce = cudaStreamEndCapture(m->st, &g);
+    if (rc != 0 || ce != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        MCK(ce);
+        return -1;
+    }
+    const cudaError_t e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    MCK(e);
+    return 0;
 }
 
 // `steps` Adam steps of batch B over the resident data set, sampled through a
@@ -968,12 +1182,8 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
     }
     if (mlp_batch_buffers(m, B) != 0) return -1;
     MCK(cudaMemsetAsync(m->step, 0, sizeof(long long), m->st));
-    m->adam_cfg.lr0 = (float)lr;
-    m->adam_cfg.beta1 = (float)beta1;
-    m->adam_cfg.beta2 = (float)beta2;
-    m->adam_cfg.eps = (float)eps;
-    m->adam_cfg.total_steps = (long long)steps;
-    m->adam_cfg.step = m->step;
+    const AdamCfg cfg = {(float)lr, (float)beta1, (float)beta2, (float)eps, (long long)steps};
+    MCK(cudaMemcpyAsync(m->cfg, &cfg, sizeof cfg, cudaMemcpyHostToDevice, m->st));
     // first and second moments restart
     for (Layer &ly : m->L) {
         MCK(cudaMemsetAsync(ly.mw, 0, (size_t)ly.out * ly.in * 4, m->st));
@@ -981,44 +1191,29 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
         MCK(cudaMemsetAsync(ly.mb, 0, ly.out * 4, m->st));
         MCK(cudaMemsetAsync(ly.vb, 0, ly.out * 4, m->st));
     }
-    if (m->graph && m->graph_b != B) {
-        cudaGraphExecDestroy(m->graph);
-        m->graph = nullptr;
-    }
-    if (m->graph) {
-        // the captured Adam arguments hold the old schedule: capture again
-        cudaGraphExecDestroy(m->graph);
-        m->graph = nullptr;
-    }
-    {
-        cudaGraph_t g = nullptr;
-        MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-        mlp_train_step(m, B);
-        MCK(cudaStreamEndCapture(m->st, &g));
-        const cudaError_t e = cudaGraphInstantiate(&m->graph, g, 0);
-        cudaGraphDestroy(g);
-        MCK(e);
-        m->graph_b = B;
-    }
+    if (m->graph_b != B) mlp_free_graphs(m);
+    m->graph_b = B;
     const size_t per_pass = std::max<size_t>(1, m->n_data / B);
     std::vector<int> perm(m->n_data);
     uint64_t rs = shuffle_seed;
     size_t done = 0;
     while (done < steps) {
-        // permutation of this pass (Fisher-Yates on splitmix64)
+        // permutation of this pass (Fisher-Yates on splitmix64), drawn while
+        // the pass before runs; the copy to the device queues behind its steps
         for (size_t q = 0; q < m->n_data; q++) perm[q] = (int)q;
         for (size_t q = m->n_data - 1; q > 0; q--) std::swap(perm[q], perm[splitmix(rs) % (q + 1)]);
         MCK(cudaMemcpyAsync(m->perm, perm.data(), m->n_data * sizeof(int), cudaMemcpyHostToDevice, m->st));
         const size_t run = std::min(per_pass, steps - done);
-        for (size_t s = 0; s < run; s++) {
-            MCK(cudaGraphLaunch(m->graph, m->st));
-            m->launches += 0;
+        for (size_t s = 0; s < run;) {
+            const bool many = run - s >= (size_t)GRAPH_STEPS;
+            cudaGraphExec_t *g = many ? &m->graph_n : &m->graph;
+            if (!*g && mlp_capture(m, B, many ? GRAPH_STEPS : 1, g) != 0) return -1;
+            MCK(cudaGraphLaunch(*g, m->st));
+            s += many ? GRAPH_STEPS : 1;
         }
-        // the permutation buffer is rewritten for the next pass only after
-        // this pass's steps have read it
-        MCK(cudaStreamSynchronize(m->st));
         done += run;
     }
+    MCK(cudaStreamSynchronize(m->st));
     if (final_loss) {
         const int nb = (B * m->n_out + 255) / 256;
         std::vector<float> part(nb);
@@ -1030,24 +1225,24 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
     return mlp_check_err(m);
 }
 
-// Network outputs of n inputs (any n; evaluated in batches of up to 1024).
+// Network outputs of n inputs (any n; evaluated in batches of up to 1024
+// rows, queued one behind the other).
 extern "C" int fdtd_b200_mlp_predict(fdtd_b200_mlp_t *m, const float *X, size_t n, float *Y) {
     const int B = 1024;
     if (mlp_batch_buffers(m, B) != 0) return -1;
-    std::vector<float> xb((size_t)B * m->n_in, 0.f);
     for (size_t r0 = 0; r0 < n; r0 += B) {
         const size_t rows = std::min<size_t>(B, n - r0);
-        std::fill(xb.begin(), xb.end(), 0.f);
-        memcpy(xb.data(), X + r0 * m->n_in, rows * m->n_in * sizeof(float));
         // rows padded to the tensor-core tile height (zero rows)
         const int Bp = (int)((rows + tc::BM - 1) / tc::BM * tc::BM);
-        if (mlp_upload_x(m, xb.data(), Bp, m->act[0]) != 0) return -1;
-        mlp_forward(m, Bp);
+        if (mlp_upload_x(m, X + r0 * m->n_in, rows, m->act[0], m->xf) != 0) return -1;
+        if ((size_t)Bp > rows)
+            MCK(cudaMemsetAsync(m->act[0] + rows * m->kin, 0, (Bp - rows) * m->kin * sizeof(bf16), m->st));
+        mlp_forward(m, Bp, false);
         MCK(cudaGetLastError());
         MCK(cudaMemcpyAsync(Y + r0 * m->n_out, m->out, rows * m->n_out * sizeof(float), cudaMemcpyDeviceToHost,
                             m->st));
-        MCK(cudaStreamSynchronize(m->st));
     }
+    MCK(cudaStreamSynchronize(m->st));
     return mlp_check_err(m);
 }
 

@@ -643,7 +643,7 @@ struct rfb_engine {
     long long *probe_cell = nullptr;
     int *probe_comp = nullptr;
     void *ts = nullptr;
-    int *d_step = nullptr;
+    int *d_step = nullptr, *d_tail_done = nullptr;
     size_t n_steps = 0, steps_done = 0;
     double *d_omega = nullptr, *d_re = nullptr, *d_im = nullptr;
     size_t dft_cap = 0;
@@ -765,21 +765,15 @@ static TfArgs<T> tf_args(const rfb_engine *e, int par) {
     return t;
 }
 
-// Plane wave: H corrections from the line's E^n, then the line's H to n+1/2
-// (before the interface list, whose boundary entries read it).
+// Plane wave: H corrections from the line's E^n, and the line's H to n+1/2
+// (before the interface list, whose boundary entries read it); k_step_tail
+// takes the line's E to n+1.
 template <typename T>
 static void tf_before_list(rfb_engine *e, int par) {
     if (!e->tf_on) return;
     TfArgs<T> t = tf_args<T>(e, par);
-    if (t.n_h) launch_step(k_tfsf_h<T>, dim3((t.n_h + 255) / 256), dim3(256), 0, e->stream, e->overlap, t);
-    launch_step(k_inc_h<T>, dim3((t.m_len + 255) / 256), dim3(256), 0, e->stream, e->overlap, t);
-}
-// ... and the line's E to n+1 after the step counter advanced.
-template <typename T>
-static void tf_after_step(rfb_engine *e, int par) {
-    if (!e->tf_on) return;
-    TfArgs<T> t = tf_args<T>(e, par);
-    launch_step(k_inc_e<T>, dim3((t.m_len + 255) / 256), dim3(256), 0, e->stream, e->overlap, t);
+    const int nb_h = (t.n_h + 255) / 256;
+    launch_step(k_tfsf_before<T>, dim3(nb_h + (t.m_len + 255) / 256), dim3(256), 0, e->stream, e->overlap, t, nb_h);
 }
 
 // Interior sweep of the plan: TMA-fed or cp.async-fed variant, or (mode 2)
@@ -887,15 +881,24 @@ static void launch_list(rfb_engine *e, const Args<T> &a) {
     }
 }
 
-// Plane probes of the step: their means join the series before the point
-// probes advance the step counter.
+// The end of the step: plane probes, point probes, the plane wave's line and
+// the step counter.
 template <typename T>
-static void launch_plane_gather(rfb_engine *e, int par) {
-    if (!e->n_planes) return;
+static void launch_tail(rfb_engine *e, int par) {
     const int out = e->nbuf == 2 ? 1 - par : 0;
-    launch_step(
-        k_plane_gather<T>, dim3(e->plane_chunks, e->n_planes), dim3(kPlaneThreads), 0, e->stream, e->overlap, e->d_planes, e->n_planes, (const T *const *)e->d_fout[out], (T *)e->ts, e->n_probes, (long long)e->n_steps,
-        e->d_step, e->d_plane_part, e->d_plane_count, e->plane_chunks);
+    ProbeArgs<T> p;
+    p.n = e->n_probes;
+    p.cell = e->probe_cell;
+    p.comp = e->probe_comp;
+    for (int c = 0; c < 6; c++) p.F[c] = (const T *)e->fld[out][c];
+    p.ts = (T *)e->ts;
+    p.n_steps = (long long)e->n_steps;
+    p.d_step = e->d_step;
+    const PlaneArgs pl = {e->d_planes, e->n_planes, std::max(1, e->plane_chunks), e->n_probes,
+                          (const void *const *)e->d_fout[out], e->d_plane_part, e->d_plane_count};
+    const int nb_line = e->tf_on ? (e->tf_m_len + kLineChunk - 1) / kLineChunk : 0;
+    launch_step(k_step_tail<T>, dim3(1 + nb_line + e->plane_chunks * e->n_planes), dim3(kPlaneThreads), 0, e->stream,
+                e->overlap, p, pl, tf_args<T>(e, par), nb_line, e->d_tail_done);
 }
 
 template <typename T>
@@ -912,18 +915,7 @@ static void enqueue_step(rfb_engine *e, int par) {
     }
     tf_before_list<T>(e, par);
     launch_list<T>(e, a);
-    ProbeArgs<T> p;
-    p.n = e->n_probes;
-    p.cell = e->probe_cell;
-    p.comp = e->probe_comp;
-    const int out = e->nbuf == 2 ? 1 - par : 0;
-    for (int c = 0; c < 6; c++) p.F[c] = (const T *)e->fld[out][c];
-    p.ts = (T *)e->ts;
-    p.n_steps = (long long)e->n_steps;
-    p.d_step = e->d_step;
-    launch_plane_gather<T>(e, par);
-    launch_step(k_probe_gather<T>, dim3(1), dim3(128), 0, e->stream, e->overlap, p);
-    tf_after_step<T>(e, par);
+    launch_tail<T>(e, par);
 }
 
 // The running DFT over the last `count` recorded samples of every series.
@@ -944,9 +936,7 @@ static int sweep_launches(const rfb_engine *e) {
 static int count_step_launches(const rfb_engine *e) {
     int n = e->sched == RFB_SCHED_FUSED ? sweep_launches(e) : 2;
     n += list_launches(e);
-    if (e->tf_on) n += 2 + (e->tf_n_h > 0);
-    if (e->n_planes) n++;
-    return n + 1;
+    return n + (e->tf_on ? 1 : 0) + 1;
 }
 
 // Programmatic links between a step's kernels: for small scenes on the vector
@@ -1885,8 +1875,10 @@ static rfb_engine_t *engine_create(const rfb_geom_t *geom, int precision, int sc
         CK(cudaMemset(e->ts, 0, n_probes * n_steps * e->esz));
         if (!e->probe_cell || !e->probe_comp) { rfb_set_error("probe upload failed"); goto fail_noset; }
     }
-    CK(dmalloc(&e->d_step, sizeof(int)));
-    CK(cudaMemset(e->d_step, 0, sizeof(int)));
+    // the step counter, then the count of finished blocks of k_step_tail
+    CK(dmalloc(&e->d_step, 2 * sizeof(int)));
+    CK(cudaMemset(e->d_step, 0, 2 * sizeof(int)));
+    e->d_tail_done = e->d_step + 1;
     CK(dmalloc(&e->d_err, sizeof(int)));
     CK(cudaMemset(e->d_err, 0, sizeof(int)));
     if (schedule == RFB_SCHED_FUSED) {
@@ -2077,7 +2069,7 @@ extern "C" int rfb_engine_reset(rfb_engine_t *e) {
     // the plane gather's counters are zero between launches; a launch cut
     // short by an error would leave them counting
     if (e->d_plane_count) CK(cudaMemsetAsync(e->d_plane_count, 0, (size_t)e->n_planes * sizeof(int), e->stream));
-    CK(cudaMemsetAsync(e->d_step, 0, sizeof(int), e->stream));
+    CK(cudaMemsetAsync(e->d_step, 0, 2 * sizeof(int), e->stream));
     e->steps_done = 0;
     e->parity = 0;
     return 0;
@@ -2190,20 +2182,9 @@ static int time_kernels_t(rfb_engine *e, size_t n, double *sweep_ms, double *oth
         tf_before_list<T>(e, par);
         launch_list<T>(e, a);
         g_launches += list_launches(e);
-        ProbeArgs<T> p;
-        p.n = e->n_probes;
-        p.cell = e->probe_cell;
-        p.comp = e->probe_comp;
-        const int out = e->nbuf == 2 ? 1 - par : 0;
-        for (int c = 0; c < 6; c++) p.F[c] = (const T *)e->fld[out][c];
-        p.ts = (T *)e->ts;
-        p.n_steps = (long long)e->n_steps;
-        p.d_step = e->d_step;
-        launch_plane_gather<T>(e, par);
-        launch_step(k_probe_gather<T>, dim3(1), dim3(128), 0, e->stream, e->overlap, p);
-        tf_after_step<T>(e, par);
+        launch_tail<T>(e, par);
         launch_dft_run<T>(e, 1);
-        g_launches += 1 + (e->tf_on ? 2 + (e->tf_n_h > 0) : 0) + (e->n_planes > 0) + dft_launches(e);
+        g_launches += 1 + (e->tf_on ? 1 : 0) + dft_launches(e);
         CK(cudaEventRecord(ev[2], e->stream));
         CK(cudaEventSynchronize(ev[2]));
         float t1 = 0.f, t2 = 0.f;

@@ -351,48 +351,88 @@ __device__ __forceinline__ T e_tensor3(const Args<T> &a, const T *r, int c, int 
     return xa(xm(r[4], v), xm(r[3], value));
 }
 
+// Which H samples around a cell its 3x3 update reads: H_f at (su, sv, sf)
+// steps along (f + 1, f + 2, f), for the curls D_{f+1} and D_{f+2} at the cell,
+// one step back along their own axis and one step on along each other axis.
+__host__ __device__ constexpr bool t3_reads(int su, int sv, int sf) {
+    auto both = [](int p, int q, int r) {
+        return p <= 0 && ((q == 0 && r == 0) || (q == 1 && r == 0) || (q == 0 && r == 1) || (q == -1 && r == 0) ||
+                          (q == -1 && r == 1));
+    };
+    return both(su, sv, sf) || both(sv, su, sf);
+}
+
 // The three components of a cell whose samples are all 3x3 samples (no
 // source, no TF/SF term): e_tensor3 for c = 0, 1, 2 with the same operation
-// order, the curl differences they share computed once -- D_b at the cell
-// and at the cell one step back along b serve both components c != b -- so
-// a cell takes 18 curl evaluations instead of 27.
+// order.  Its 18 curl differences read 36 H samples, 12 a component, 72
+// times: each is loaded once.  The list of the 128 x 128 x 512 unit cell is
+// bound by the latency and the bytes of its gathers (213 MB a step, 3.7 TB/s,
+// cold) rather than by their number: 56.6 -> 55.4 us a step.
 template <typename T>
 __device__ __forceinline__ void t3_cell(const Args<T> &a, int cell) {
-    const int i = a.lc_ijk[3 * cell], j = a.lc_ijk[3 * cell + 1], k = a.lc_ijk[3 * cell + 2];
+    const int p[3] = {a.lc_ijk[3 * cell], a.lc_ijk[3 * cell + 1], a.lc_ijk[3 * cell + 2]};
+    const int tix[3] = {a.l_tix[3 * cell], a.l_tix[3 * cell + 1], a.l_tix[3 * cell + 2]};
     const int n[3] = {a.nx, a.ny, a.nz};
     const long long st[3] = {(long long)(a.ny + 1) * a.pitch, a.pitch, 1};
-    auto curl_at = [&](int b, long long q, const int p[3]) {
-        const int fa = (b + 2) % 3, axa = (b + 1) % 3, fb = (b + 1) % 3, axb = (b + 2) % 3;
-        const long long qa = p[axa] == 0 ? q + (long long)(n[axa] - 1) * st[axa] : q - st[axa];
-        const long long qb = p[axb] == 0 ? q + (long long)(n[axb] - 1) * st[axb] : q - st[axb];
-        return xs(xs(a.Ho[fa][q], a.Ho[fa][qa]), xs(a.Ho[fb][q], a.Ho[fb][qb]));
-    };
-    const int p0[3] = {i, j, k};
-    const long long c0 = cidx(a, i, j, k);
-    T dw[3], dm[3];
-    long long back[3];
-    for (int b = 0; b < 3; b++) {
-        dw[b] = curl_at(b, c0, p0);
-        int p2[3] = {i, j, k};
-        p2[b] = p2[b] == 0 ? n[b] - 1 : p2[b] - 1;
-        back[b] = p0[b] == 0 ? (long long)(n[b] - 1) * st[b] : -st[b];
-        dm[b] = curl_at(b, c0 + back[b], p2);
+    const long long c0 = cidx(a, p[0], p[1], p[2]);
+    // element offsets of one step back and one step on along each axis: a
+    // step back from 0 wraps (periodic axes only: elsewhere the host admits
+    // samples in [1, n-1]), a step on wraps on periodic axes
+    long long o[3][3];
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        o[x][0] = p[x] == 0 ? (long long)(n[x] - 1) * st[x] : -st[x];
+        o[x][1] = 0;
+        o[x][2] = ((a.per >> x) & 1u) && p[x] + 1 == n[x] ? -(long long)(n[x] - 1) * st[x] : st[x];
     }
+    T h[3][3][3][3];  // [f][su + 1][sv + 1][sf + 1], the samples t3_reads names
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+#pragma unroll
+        for (int su = -1; su <= 1; su++)
+#pragma unroll
+            for (int sv = -1; sv <= 1; sv++)
+#pragma unroll
+                for (int sf = -1; sf <= 1; sf++)
+                    if (t3_reads(su, sv, sf))
+                        h[f][su + 1][sv + 1][sf + 1] =
+                            __ldg(a.Ho[f] + (c0 + o[(f + 1) % 3][su + 1] + o[(f + 2) % 3][sv + 1] + o[f][sf + 1]));
+    T e[3], r[3][5];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-        const T *r = a.t3 + 5 * (long long)a.l_tix[3 * cell + c];
-        T value = xm(r[c], dw[c]);
-        const bool wrap = ((a.per >> c) & 1u) && p0[c] + 1 == n[c];
-        int p1[3] = {i, j, k};
-        p1[c] = wrap ? 0 : p1[c] + 1;
-        const long long c1 = wrap ? c0 - (long long)(n[c] - 1) * st[c] : c0 + st[c];
+        e[c] = __ldg(a.E[c] + c0);
+#pragma unroll
+        for (int q = 0; q < 5; q++) r[c][q] = __ldg(a.t3 + 5 * (long long)tix[c] + q);
+    }
+    // H_f at the cell moved by d (steps per axis)
+    auto H = [&](int f, int dx, int dy, int dz) {
+        const int d[3] = {dx, dy, dz};
+        return h[f][d[(f + 1) % 3] + 1][d[(f + 2) % 3] + 1][d[f] + 1];
+    };
+    // D_b at the cell moved by d: (H_{b+2}(w) - H_{b+2}(w - e_{b+1})) -
+    // (H_{b+1}(w) - H_{b+1}(w - e_{b+2}))
+    auto curl = [&](int b, int dx, int dy, int dz) {
+        const int u = (b + 1) % 3, v = (b + 2) % 3;
+        return xs(xs(H(v, dx, dy, dz), H(v, dx - (u == 0), dy - (u == 1), dz - (u == 2))),
+                  xs(H(u, dx, dy, dz), H(u, dx - (v == 0), dy - (v == 1), dz - (v == 2))));
+    };
+    T dw[3], dm[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        dw[b] = curl(b, 0, 0, 0);
+        dm[b] = curl(b, -(b == 0), -(b == 1), -(b == 2));
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        T value = xm(r[c][c], dw[c]);
+#pragma unroll
         for (int b = 0; b < 3; b++) {
             if (b == c) continue;
-            int p3[3] = {p1[0], p1[1], p1[2]};
-            p3[b] = p3[b] == 0 ? n[b] - 1 : p3[b] - 1;
-            const T s4 = xa(xa(xa(dw[b], curl_at(b, c1, p1)), dm[b]), curl_at(b, c1 + back[b], p3));
-            value = xa(value, xm(r[b], xm(T(0.25), s4)));
+            const T s4 = xa(xa(xa(dw[b], curl(b, c == 0, c == 1, c == 2)), dm[b]),
+                            curl(b, (c == 0) - (b == 0), (c == 1) - (b == 1), (c == 2) - (b == 2)));
+            value = xa(value, xm(r[c][b], xm(T(0.25), s4)));
         }
-        a.Eo[c][c0] = xa(xm(r[4], a.E[c][c0]), xm(r[3], value));
+        a.Eo[c][c0] = xa(xm(r[c][4], e[c]), xm(r[c][3], value));
     }
 }
 
@@ -499,45 +539,28 @@ struct TfArgs {
     long long n_steps;
 };
 
-// H samples next to the boundary: H += coef * interp(E1D around idx) for
-// each of their terms, in order (E1D at step n).
+// Before the interface list, in one launch: the first nb_h blocks correct the
+// H samples next to the boundary, H += coef * interp(E1D around idx) for each
+// of their terms, in order (E1D at step n); the others take the line's H to
+// n + 1/2, H1D[m] -= ch (E1D[m+1] - E1D[m]).  Neither reads what the other
+// writes.
 template <typename T>
-__global__ void k_tfsf_h(TfArgs<T> a) {
+__global__ void __launch_bounds__(256) k_tfsf_before(TfArgs<T> a, int nb_h) {
     grid_launch_next();
     grid_wait();
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.n_h) return;
-    T *f = a.Ho[a.h_comp[q]] + a.h_cell[q];
-    T h = *f;
-    for (int t = a.h_first[q]; t < a.h_first[q] + a.h_count[q]; t++) {
-        const int m = a.h_idx[t];
-        h = xa(h, xm(a.h_coef[t], tf_interp(a.h_w + 4 * t, a.inc_e + m)));
-    }
-    *f = h;
-}
-
-// The line's H: H1D[m] -= ch (E1D[m+1] - E1D[m]).
-template <typename T>
-__global__ void k_inc_h(TfArgs<T> a) {
-    grid_launch_next();
-    grid_wait();
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < a.m_len - 1; m += gridDim.x * blockDim.x)
-        a.inc_h[m] = xs(a.inc_h[m], xm(a.ch, xs(a.inc_e[m + 1], a.inc_e[m])));
-}
-
-// The line's E: E1D[m] -= ce (H1D[m] - H1D[m-1]); E1D[0] is the hard source
-// of the step just completed (the step counter already advanced).
-template <typename T>
-__global__ void k_inc_e(TfArgs<T> a) {
-    grid_launch_next();
-    grid_wait();
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < a.m_len - 1; m += gridDim.x * blockDim.x) {
-        if (m == 0) {
-            const long long n = *a.d_step;
-            a.inc_e[0] = a.src[n < a.n_steps ? n : a.n_steps];
-        } else {
-            a.inc_e[m] = xs(a.inc_e[m], xm(a.ce, xs(a.inc_h[m], a.inc_h[m - 1])));
+    if ((int)blockIdx.x < nb_h) {
+        const int q = blockIdx.x * 256 + threadIdx.x;
+        if (q >= a.n_h) return;
+        T *f = a.Ho[a.h_comp[q]] + a.h_cell[q];
+        T h = *f;
+        for (int t = a.h_first[q]; t < a.h_first[q] + a.h_count[q]; t++) {
+            const int m = a.h_idx[t];
+            h = xa(h, xm(a.h_coef[t], tf_interp(a.h_w + 4 * t, a.inc_e + m)));
         }
+        *f = h;
+    } else {
+        const int m = (blockIdx.x - nb_h) * 256 + threadIdx.x;
+        if (m < a.m_len - 1) a.inc_h[m] = xs(a.inc_h[m], xm(a.ch, xs(a.inc_e[m + 1], a.inc_e[m])));
     }
 }
 
@@ -562,8 +585,9 @@ __global__ void __launch_bounds__(256) k_e_list(Args<T> a) {
 // so running them side by side changes no result, and their dependent
 // gathers overlap instead of ending one launch before the next begins.
 // The kernel is bound by the latency of those gathers, so in FP32 it is
-// held to 40 registers (6 blocks of 256 per SM, against 4 at its natural
-// 60; 32 bytes of spills): C3's step 0.2233 -> 0.2181 ms, C2's ~1 % faster.
+// held to 40 registers (6 blocks of 256 per SM; 68 bytes of spills) against
+// 64 at 4: the unit cell's list 55.4 against 53.5 us, but that of the 256^3
+// scene, whose entries are scattered scalar samples, 20 against 26 us.
 // FP64 keeps the 3 blocks per SM of its natural 78-80 registers.
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 3) k_list_cells(Args<T> a, const int *t3, int n_t3, int nb_t3, const int *ade,
@@ -595,34 +619,17 @@ struct ProbeArgs {
     int *d_step;
 };
 
-// Records sample n of every probe after the step, then advances the device
-// step counter (single block).
-template <typename T>
-__global__ void k_probe_gather(ProbeArgs<T> p) {
-    __shared__ int n;
-    grid_launch_next();
-    grid_wait();
-    if (threadIdx.x == 0) n = *p.d_step;
-    __syncthreads();
-    if (n < p.n_steps)
-        for (int q = threadIdx.x; q < p.n; q += blockDim.x)
-            p.ts[(long long)q * p.n_steps + n] = p.F[p.comp[q]][p.cell[q]];
-    __syncthreads();
-    if (threadIdx.x == 0) *p.d_step = n + 1;
-}
-
 // ---- plane probes ------------------------------------------------------------
 // Sample n of a plane probe is the mean of one field component over a whole
 // grid plane (axis a at index q: every (u, v) of the other two axes, u < n_u,
 // v < n_v): for a periodic cell at normal incidence, the amplitude of the
 // specular (zeroth-order) reflected or transmitted wave.  The plane's points
-// t = u n_v + v are cut into chunks of kPlaneChunk, one block each (grid:
-// chunks x planes), so the gather spreads over the SMs.  Each thread sums
+// t = u n_v + v are cut into chunks of kPlaneChunk, one block each, so the gather spreads over the SMs.  Each thread sums
 // its points of the chunk (t0 + x, t0 + x + kPlaneThreads, ...) in FP64,
 // warp shuffles and one pass over the warps' sums reduce the block in a
 // fixed tree, and the last block of the plane to finish (a per-plane
 // counter, reset by that block) adds the chunks' sums in chunk order: the
-// mean is deterministic.  Runs before k_probe_gather (same step index).
+// mean is deterministic.
 struct PlaneDesc {
     long long base, su, sv;  // element offset of (u, v) = (0, 0) and the strides
     int nu, nv, comp;
@@ -630,47 +637,80 @@ struct PlaneDesc {
 
 constexpr int kPlaneChunk = 1024, kPlaneThreads = 256;
 
+struct PlaneArgs {
+    const PlaneDesc *planes;
+    int n, max_chunks, series0;
+    const void *const *F;  // the six output components
+    double *part;
+    int *count;            // per plane, zero between launches
+};
+constexpr int kLineChunk = 4 * kPlaneThreads;  // points of the plane wave's line a block takes
+
+// The end of a step in one launch.  Block 0 records sample n of every point
+// probe; the next nb_line blocks, with a plane wave, take its line's E to n + 1
+// (E1D[m] -= ce (H1D[m] - H1D[m-1]); E1D[0] is the hard source of the step
+// just completed); the others take the plane probes' chunks.  Every block has
+// read the step counter before it counts itself off in *done (zero between
+// launches); the last one advances it.
 template <typename T>
-__global__ void __launch_bounds__(kPlaneThreads) k_plane_gather(const PlaneDesc *planes, int n_planes,
-                                                                const T *const *F, T *ts, int series0,
-                                                                long long n_steps, const int *d_step, double *part,
-                                                                int *count, int max_chunks) {
+__global__ void __launch_bounds__(kPlaneThreads) k_step_tail(ProbeArgs<T> p, PlaneArgs pl, TfArgs<T> tf, int nb_line,
+                                                             int *done) {
     __shared__ double warp_sum[kPlaneThreads / 32];
     grid_launch_next();
     grid_wait();
-    const int q = blockIdx.y, b = blockIdx.x;
-    if (q >= n_planes) return;
-    const int n = *d_step;
-    if (n >= n_steps) return;
-    const PlaneDesc pd = planes[q];
-    const long long npts = (long long)pd.nu * pd.nv;
-    const int nchunk = (int)((npts + kPlaneChunk - 1) / kPlaneChunk);
-    if (b >= nchunk) return;
-    const T *f = F[pd.comp];
-    const long long t0 = (long long)b * kPlaneChunk, t1 = t0 + kPlaneChunk < npts ? t0 + kPlaneChunk : npts;
-    double acc = 0.0;
-    for (long long t = t0 + threadIdx.x; t < t1; t += kPlaneThreads) {
-        const long long u = t / pd.nv, v = t - u * pd.nv;
-        acc = __dadd_rn(acc, (double)f[pd.base + u * pd.su + v * pd.sv]);
-    }
-    for (int off = 16; off > 0; off >>= 1) acc = __dadd_rn(acc, __shfl_down_sync(0xffffffffu, acc, off));
-    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < kPlaneThreads / 32; w++) s = __dadd_rn(s, warp_sum[w]);
-        part[(long long)q * max_chunks + b] = s;
-        __threadfence();
-        if (atomicAdd(&count[q], 1) == nchunk - 1) {
-            // every chunk's sum is visible: the other blocks fenced before
-            // their increments
-            __threadfence();
-            const volatile double *pp = part + (long long)q * max_chunks;
-            double m = 0.0;
-            for (int c = 0; c < nchunk; c++) m = __dadd_rn(m, pp[c]);
-            ts[(long long)(series0 + q) * n_steps + n] = (T)__ddiv_rn(m, (double)npts);
-            count[q] = 0;
+    const int n = *p.d_step, tid = threadIdx.x;
+    if (blockIdx.x == 0) {
+        if (n < p.n_steps)
+            for (int q = tid; q < p.n; q += kPlaneThreads)
+                p.ts[(long long)q * p.n_steps + n] = p.F[p.comp[q]][p.cell[q]];
+    } else if ((int)blockIdx.x <= nb_line) {
+        const int m0 = (blockIdx.x - 1) * kLineChunk, m1 = min(m0 + kLineChunk, tf.m_len - 1);
+        for (int m = m0 + tid; m < m1; m += kPlaneThreads) {
+            if (m == 0) tf.inc_e[0] = tf.src[n + 1 < tf.n_steps ? n + 1 : tf.n_steps];
+            else tf.inc_e[m] = xs(tf.inc_e[m], xm(tf.ce, xs(tf.inc_h[m], tf.inc_h[m - 1])));
         }
+    } else {
+        const int blk = blockIdx.x - 1 - nb_line, q = blk / pl.max_chunks, b = blk % pl.max_chunks;
+        const PlaneDesc pd = pl.planes[q];
+        const long long npts = (long long)pd.nu * pd.nv;
+        const int nchunk = (int)((npts + kPlaneChunk - 1) / kPlaneChunk);
+        if (n < p.n_steps && b < nchunk) {
+            const T *f = static_cast<const T *>(pl.F[pd.comp]);
+            const long long t0 = (long long)b * kPlaneChunk, t1 = t0 + kPlaneChunk < npts ? t0 + kPlaneChunk : npts;
+            double acc = 0.0;
+            for (long long t = t0 + tid; t < t1; t += kPlaneThreads) {
+                const long long u = t / pd.nv, v = t - u * pd.nv;
+                acc = __dadd_rn(acc, (double)f[pd.base + u * pd.su + v * pd.sv]);
+            }
+            for (int off = 16; off > 0; off >>= 1) acc = __dadd_rn(acc, __shfl_down_sync(0xffffffffu, acc, off));
+            if ((tid & 31) == 0) warp_sum[tid >> 5] = acc;
+            __syncthreads();
+            if (tid == 0) {
+                double s = 0.0;
+                for (int w = 0; w < kPlaneThreads / 32; w++) s = __dadd_rn(s, warp_sum[w]);
+                pl.part[(long long)q * pl.max_chunks + b] = s;
+                __threadfence();
+                if (atomicAdd(&pl.count[q], 1) == nchunk - 1) {
+                    // every chunk's sum is visible: the other blocks fenced before
+                    // their increments
+                    __threadfence();
+                    const volatile double *pp = pl.part + (long long)q * pl.max_chunks;
+                    double m = 0.0;
+                    for (int c = 0; c < nchunk; c++) m = __dadd_rn(m, pp[c]);
+                    p.ts[(long long)(pl.series0 + q) * p.n_steps + n] = (T)__ddiv_rn(m, (double)npts);
+                    pl.count[q] = 0;
+                }
+            }
+        }
+    }
+    __syncthreads();  // every thread has read the counter
+    if (tid == 0) {
+        if (gridDim.x > 1) {
+            __threadfence();
+            if (atomicAdd(done, 1) != (int)gridDim.x - 1) return;
+            *done = 0;
+        }
+        *p.d_step = n + 1;
     }
 }
 

@@ -1286,16 +1286,27 @@ static int v_max_seg(const rfb_engine *e) {
     return (int)std::min<long long>(((1LL << 32) - 1) / plane - 1, 1 << 20);
 }
 
-// Tile shape and segment length.  A CTA takes about the same time a plane
-// however small its tile (the plane's chain of dependent instructions, 1.1-
-// 1.4 us on B200), so the rule minimises the planes the busiest CTA slot
-// marches, one more than its length per item: segments that give one wave of
-// CTAs where that takes at most 16 planes each (small grids), else two waves
-// or more of at most 32 planes, which balance the slab items; of all shapes,
-// the one whose march, weighted with its halo threads, is shortest.  Against
-// 24 shapes a grid, on 18 grids of 48^3-256^3, odd extents and both
-// precisions, the rule's pick is on average 3 % and at most 11 % slower than
-// the fastest.
+// Tile shape and segment length, by the planes W that a CTA slot gets.
+//
+// Large grids (W > V_DENSE): CTAs of at most 128 threads, three to an SM, that
+// leave each other's barriers alone, on tiles 8 vectors wide where the grid
+// allows: their rows are whole 128-byte lines, so no two CTAs write parts of
+// one.  Of such shapes (13 x 8 on most grids) the one with the fewest tiles,
+// others counting 1.1 (measured 1.02-1.1).  Segments of three quarters of W,
+// at least 8 and at most 28 planes: shorter ones march more halo planes,
+// longer ones leave slots empty at the end.  Sweep alone, against the small
+// grids' rule: 256^3 FP32 238 for 245 us, a 128 x 128 x 512 unit cell 104 for
+// 118, 150 x 131 x 170 FP64 112 for 124, 150^3 FP32 64 for 80, 128^3 49 for
+// 56, 112^3 40 for 50, 96^3 FP64 44 for 52, 90^3 FP64 (W = 8.2) 40 for 42.
+//
+// Small grids: a CTA takes about the same time a plane however small its tile
+// (the plane's chain of dependent instructions, 1.1-1.4 us), so the rule
+// minimises the planes the busiest slot marches, one more than its length per
+// item, weighted with the halo threads of the shape: 96^3 FP32 (W = 5) 29.9 us
+// for 31.6 on 13 x 8, 200 x 200 x 30 (W = 7.2) the same on both.  Where y is
+// periodic, no slab planes contend and the line lies higher: 77 x 91 x 203
+// (W = 8.5) 26.8 for 28.0, 96 x 96 x 203 (W = 12) 35.0 for 34.7 the other way.
+constexpr double V_DENSE = 8.0, V_DENSE_PY = 10.0;
 constexpr int V_REGS = 168;  // registers a thread of k_vsweep holds at most
 
 struct VPick {
@@ -1319,6 +1330,28 @@ static void v_x_range(const rfb_engine *e, int *xa, int *xb) {
 
 static VPick v_rule(const rfb_engine *e, int cj, int ck, int ci) {
     const int N = e->prec == RFB_FP64 ? 2 : 4, nvk = (ck + N - 1) / N, sms = 148;
+    {
+        VPick d = {0, 0, 0, 0};
+        double cost = 1e300, w = 0;
+        for (int nv = 1; nv <= nvk; nv++) {
+            const int most = std::min(cj, 128 / (nv + 1) - 1);
+            if (most < 1) break;
+            const int nj = (cj + most - 1) / most, tr = (cj + nj - 1) / nj;
+            VShape s;
+            if (!v_layout(e, s, nv, tr, cj, ck)) continue;
+            const double tiles = (double)((nvk + nv - 1) / nv) * nj, c = tiles * (nv % 8 ? 1.1 : 1.0);
+            if (c < cost) {
+                cost = c;
+                w = tiles * ci / ((double)sms * v_slots(s.nt, s.smem));
+                d.tr = tr;
+                d.nv = nv;
+            }
+        }
+        if (w > ((e->g.periodic & 2u) ? V_DENSE_PY : V_DENSE)) {
+            d.seg_int = d.seg_edge = (int)std::min(28.0, std::max(8.0, ceil(0.75 * w)));
+            return d;
+        }
+    }
     int xa, xb;
     v_x_range(e, &xa, &xb);
     const int len[3] = {std::min(xa, ci), xb - xa, std::max(0, ci - xb)};

@@ -669,17 +669,21 @@ fail:
     return nullptr;
 }
 
+static int batch_report(int err) {
+    if (err) {
+        rfb_set_error("batch: %s", sweep_error_text(err));
+        return -1;
+    }
+    return 0;
+}
+
 static int batch_check_error(rfb_batch *b) {
     int err = 0;
     if (cudaMemcpy(&err, b->d_err, sizeof err, cudaMemcpyDeviceToHost) != cudaSuccess) {
         rfb_set_error("batch: %s", cudaGetErrorString(cudaGetLastError()));
         return -1;
     }
-    if (err) {
-        rfb_set_error("batch: %s", sweep_error_text(err));
-        return -1;
-    }
-    return 0;
+    return batch_report(err);
 }
 
 extern "C" int rfb_batch_advance(rfb_batch_t *b, size_t n) {
@@ -715,10 +719,19 @@ fail:
 }
 
 extern "C" int rfb_batch_sync(rfb_batch_t *b) {
+    int err = 0;  // comes back behind the stream's work
+    CK(cudaMemcpyAsync(&err, b->d_err, sizeof err, cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    return batch_check_error(b);
+    return batch_report(err);
 fail:
     return -1;
+}
+
+// A scene's series: the batch's sweeps are the only ones that ran on it, so
+// the batch's wait and check cover it.
+extern "C" int rfb_batch_read_probes(rfb_batch_t *b, size_t scene, double *out) {
+    if (rfb_batch_sync(b) != 0) return -1;
+    return copy_series(b->m[scene], out);
 }
 
 extern "C" int rfb_batch_advance_timed(rfb_batch_t *b, size_t n, double *ms) {

@@ -152,6 +152,7 @@ int rfb_batch_reset(rfb_batch_t *b);
 int rfb_batch_advance(rfb_batch_t *b, size_t n);
 int rfb_batch_advance_timed(rfb_batch_t *b, size_t n, double *ms);
 int rfb_batch_sync(rfb_batch_t *b);
+int rfb_batch_read_probes(rfb_batch_t *b, size_t scene, double *out);
 int rfb_batch_time_kernels(rfb_batch_t *b, size_t n, double *sweep_ms, double *other_ms);
 rfb_engine_t *rfb_batch_member(rfb_batch_t *b, size_t s);
 size_t rfb_batch_size(rfb_batch_t *b);

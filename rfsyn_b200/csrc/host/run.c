@@ -909,8 +909,7 @@ int fdtd_b200_batch_read_probes(fdtd_b200_batch_t *bt, size_t scene, double *pro
         rfb_set_error("batch: bad scene index or output");
         return -1;
     }
-    if (rfb_batch_sync(bt->b) != 0) return -1;
-    return rfb_engine_read_probes(bt->sims[scene]->eng, probe_td);
+    return rfb_batch_read_probes(bt->b, scene, probe_td);
 }
 
 int fdtd_b200_batch_read_iq(fdtd_b200_batch_t *bt, size_t scene, size_t probe, const fdtd_b200_awgn_t *awgn,

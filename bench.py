@@ -37,7 +37,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 PEAKS = ROOT / "MEASURED_PEAKS.json"
-TRAFFIC = ROOT / "profiles" / "sweep_queue_c2.md"
+TRAFFIC = ROOT / "profiles" / "sweep_vector_c2.md"
 METRIC = "Mcell-updates/s"
 
 
@@ -47,6 +47,7 @@ SWEEP_KERNEL = {
     2: "k_sweep_q (one H+E sweep: interior + x-slab + edge launches)",
     3: "k_sweep_q (one H+E sweep: interior + x-slab + edge launches, shifted tiles)",
     4: "k_sweep_q (one H+E sweep: interior + x-slab + edge launches, narrow z-slab tiles)",
+    5: "k_vsweep (one H+E sweep of vector cells, one launch)",
 }
 
 
@@ -389,7 +390,7 @@ def run_b200(args) -> None:
     peak, peak_kind = hbm_peak()
     achieved = alg / (sweep_launch_ms / 1e3) / 1e9
     # the committed ncu capture covers the C2 scene's queue sweep only
-    traffic = ncu_traffic_per_launch() if args.workload == "c2" and info.tma >= 2 else None
+    traffic = ncu_traffic_per_launch() if args.workload == "c2" and info.tma == 5 else None
     sim.close()
 
     # end to end through the C ABI with host buffers: setup on the host,
@@ -456,7 +457,7 @@ def run_b200(args) -> None:
                    "list_cells": info.list_cells, "dispersive_samples": info.dispersive,
                    "schedule": "fused" if info.schedule == rb.FUSED else "split", "tile_j": info.tile_j,
                    "sweep_mode": {0: "cp.async", 1: "tma-interior", 2: "tma-queue", 3: "tma-queue-shifted",
-                                  4: "tma-queue-narrow-z"}.get(info.tma),
+                                  4: "tma-queue-narrow-z", 5: "tma-vector"}.get(info.tma),
                    "ring_depth": info.ring_depth, "single_queue": bool(info.unified),
                    "seg_len": info.seg_len, "seg_edge": info.seg_edge, "two_rows_ring": info.interior_ring2,
                    "plan": f"{info.tile_j},{info.ring_depth},{info.seg_len},{info.seg_edge},{info.tma},"

@@ -206,9 +206,11 @@ typedef struct {
     int precision, schedule;
     int tile_j, seg_len;     /* fused sweep plan: rows per interior tile, planes per work item */
     int ring_depth;          /* planes staged per interior CTA */
-    int tma;                 /* 1: interior planes staged by the Tensor Memory Accelerator */
-    int interior_items;      /* work items of the interior sweep (CTAs per step) */
-    int edge_items;          /* work items of the edge sweep */
+    int tma;                 /* sweep mode: 5 vector cells (tile_j rows x ring_depth vectors of 16
+                                bytes), 2-4 work-queue sweeps, 1 interior planes staged by TMA, 0
+                                by cp.async */
+    int interior_items;      /* work items of the interior (mode 5: items without slab or boundary cells) */
+    int edge_items;          /* the other work items */
     int unified;             /* 1: every sweep item in one work queue, one launch per step */
     int interior_ring2;      /* 0, or the ring depth of the interior sweep whose threads own two
                                 rows of a 2 tile_j-row tile */
@@ -247,15 +249,14 @@ int fdtd_b200_sim_energy(fdtd_b200_sim_t *sim, int x_lo, int x_hi, fdtd_b200_ene
  * the other (cli/main.c:362-417).  A batch uploads many scenes -- each with
  * its own size, CPML, materials (setup callback), sources and probes, as for
  * fdtd_b200_sim_create -- and advances all of them together: every step is
- * five kernel launches for the whole batch (three work-queue sweeps over the
- * tiles of every scene, the interface lists, the probes), replayed from CUDA
- * graphs.  Every scene yields exactly the probe series and spectra of its own
+ * three kernel launches for the whole batch (one sweep over the tiles of every
+ * scene, the interface lists, the probes), replayed from CUDA graphs.  Every scene yields exactly the probe series and spectra of its own
  * session (the same kernels, the same arithmetic).  All scenes share the
  * precision and step count; the FUSED schedule is used whatever the
  * configuration says; a scene periodic in y or z whose tile halos would wrap
- * is rejected.  Creation times candidate tile plans on the batch
- * (RFSYN_FDTD_PLAN "rows,ring,seg_interior,seg_edge,mode" with mode 2 or 3
- * fixes one).  setups / contexts may be NULL, or hold NULL entries. */
+ * is rejected.  The tile plan follows from the scenes' sizes; RFSYN_FDTD_PLAN
+ * fixes one: "threads,stages,seg,seg,5", or a work-queue sweep's
+ * "rows,ring,seg_interior,seg_edge,mode,single" with mode 2 to 4.  setups / contexts may be NULL, or hold NULL entries. */
 typedef struct fdtd_b200_batch fdtd_b200_batch_t;
 
 fdtd_b200_batch_t *fdtd_b200_batch_create(size_t n_scenes, const fdtd_b200_config_t *configs,
@@ -327,7 +328,7 @@ int fdtd_b200_mlp_predict(fdtd_b200_mlp_t *mlp, const float *X, size_t n, float 
 unsigned long long fdtd_b200_mlp_launch_count(const fdtd_b200_mlp_t *mlp);
 /* How many of those launches were products on the tcgen05 tensor cores
  * (accumulators in tensor memory).  The products run on mma.sync tiles of
- * 64 x 64, faster on this network's small products; with the environment
+ * 32 x 32, faster on this network's small products; with the environment
  * variable RFSYN_FDTD_MLP_GEMM=tcgen05 set when the network is created,
  * every product whose rows are a multiple of 128, columns of 32 and depth
  * of 64 runs on tcgen05 tiles of 128 x 32 instead. */
@@ -544,8 +545,9 @@ void fdtd_b200_release_cached_memory(void);
  *   precision  fp32 | fp64          default precision of rfsyn's entry points
  *   schedule   fused | split        default schedule of rfsyn's entry points
  *   plan       auto | tj,ns,seg_interior,seg_edge[,mode[,single_queue[,two_rows_ring]]]
- *                                   the sweep plan (auto = the autotuner)
- *   tune       true | false         false: the first tensor-copy variant, no tuning
+ *                                   the sweep plan (auto = by rule, or the autotuner for
+ *                                   grids periodic in z)
+ *   tune       true | false         false: never time candidate plans
  *   trace      true | false         per-phase host times on stderr
  * "default" restores a setting's initial state (its RFSYN_FDTD_* environment
  * variable decides).  Returns 0, or -1 with fdtd_b200_last_error() for an

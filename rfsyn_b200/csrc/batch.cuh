@@ -7,20 +7,17 @@
 // its own buffers (an engine created as a batch member: fields, slab psi,
 // codes, interface list, sources, probes) and advances all of them with the
 // same launches per step:
-//   k_sweep_qb<KIND 0, 1> and k_sweep_qb<KIND 2> -- the work-queue sweeps of
-//     sweep.cuh over queues of (scene, tile, plane range) items of every
-//     scene, or with the single-queue plan one k_sweep_qb<KIND 5> over every
-//     item; a CTA switching scenes copies the scene's parameters (Args) and
-//     (Ca, Cb) table into shared memory;
+//   k_vsweep_b -- the vector sweep (vsweep.cuh) over (scene, tile, plane
+//     range) items of every scene, each CTA copying its scene's parameters
+//     (Args) into shared memory; under a plan override k_sweep_qb, the
+//     work-queue sweeps of sweep.cuh over queues of such items;
 //   k_e_list_b -- the interface-list entries of every scene, one block per
 //     256 entries of one scene;
 //   k_probe_gather_b -- every probe of every scene, then the shared step
 //     counter.
-// Steps are captured in CUDA graphs (16 steps per graph), and the tile
-// height, ring depth, tile origins and segment lengths are chosen by timing
-// candidate plans on the batch itself.  Scenes whose tile halos would wrap
-// around a periodic y or z axis are not admitted (their tiles need the
-// cp.async edge sweep, which takes one scene per launch).
+// Steps are captured in CUDA graphs (16 steps per graph); tile shapes and the
+// segment length follow from the scenes' sizes (batch_build_vplan).  Scenes
+// whose tile halos would wrap around a periodic y or z axis are not admitted.
 #pragma once
 
 namespace rfb {
@@ -271,8 +268,11 @@ static void batch_free_plan(rfb_batch *b) {
 
 // Plan of mode 5, the vector sweep of every scene in one launch: per scene
 // the tile of at most `threads` threads that spends the fewest threads on the
-// grid, and one segment length for the batch by the rule of v_rule.  Items
-// of one kind together, the costly kinds first.
+// grid, and one segment length for the batch: one wave of CTAs where that
+// takes at most 16 planes each, else waves of at most 32.  Items of one kind
+// together, the costly kinds first.  96 scenes of 32-96 cells an axis, FP32:
+// 68.5 ms for 96 steps; with 128 threads 68.4-84 (segments of 32-6), with 192
+// and 12-32 planes 72.1-68.8.
 static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
     batch_free_plan(b);
     const size_t n = b->m.size();

@@ -1947,9 +1947,10 @@ static rfb_engine_t *engine_create(const rfb_geom_t *geom, int precision, int sc
             rfb_set_error("cannot configure the TMA sweep kernels' shared memory");
             goto fail_noset;
         }
-        // plan: "tj,ns,seg_interior,seg_edge[,mode[,single_queue[,i2]]]" from RFSYN_FDTD_PLAN,
-        // the autotuner (default) or, with RFSYN_FDTD_TUNE=0, the first
-        // TMA variant
+        // plan: "tj,ns,seg_interior,seg_edge[,mode[,single_queue[,i2]]]" from
+        // RFSYN_FDTD_PLAN; else the vector sweep by rule where it fits, for
+        // other grids (periodic z) the autotuner or, with RFSYN_FDTD_TUNE=0,
+        // the first TMA variant
         const char *ov = rfb_plan_override();
         int a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0, a7 = 0;
         int rc;

@@ -55,7 +55,7 @@ int fdtd_b200_set_default_schedule(int schedule) {
  * a boolean.  These are the process-wide ones; the per-run ones (DFT bins,
  * batching, per-example scenes) are read by the job runner above the ABI. */
 static char g_plan[96];
-static int g_plan_set = 0;  /* 0: RFSYN_FDTD_PLAN decides; 1: g_plan ("" = autotune) */
+static int g_plan_set = 0;  /* 0: RFSYN_FDTD_PLAN decides; 1: g_plan ("" = auto) */
 static int g_tune = -1;     /* -1: RFSYN_FDTD_TUNE decides */
 
 const char *rfb_plan_override(void) { return g_plan_set ? (g_plan[0] ? g_plan : NULL) : getenv("RFSYN_FDTD_PLAN"); }

@@ -4,8 +4,8 @@
 // same operation order, every multiply and add rounded separately through
 // __dmul_rn/__dadd_rn so nothing is contracted into an FMA) and FP32 (the
 // same order, rounded separately through __fmul_rn/__fadd_rn: every sweep
-// variant the autotuner may pick yields bit-identical FP32 fields, so runs
-// are reproducible whatever variant a process picks).
+// variant yields bit-identical FP32 fields, so runs are reproducible whatever
+// variant a process picks).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

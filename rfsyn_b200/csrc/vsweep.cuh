@@ -18,13 +18,14 @@
 // vector 0 are the tile's low-j / low-k halo: their threads recompute the
 // neighbours' H (never stored) with the same code as everyone else, so no
 // warp has an extra job.  NV and TR are run-time numbers chosen by the host
-// to divide the grid evenly (v_shape), so odd extents leave few idle lanes.
+// for the grid (v_rule), so odd extents leave few idle lanes.
 //
 // Per plane: one thread issues one tiled TMA load for E (TR + 2 rows x NV + 2
 // vectors x 3 components: the components of a buffer are one tensor) and one
-// for H (TR + 1 x NV + 1 x 3) into rings of three E and two H stages; E of plane n + 1 and H of plane n complete on one mbarrier and are
-// issued two planes ahead, right after the block barrier that frees their
-// slots.  H of the plane follows from shared E; its rows and its vectors'
+// for H (TR + 1 x NV + 1 x 3) into rings of three E and two H stages; E of
+// plane n + 1 and H of plane n complete on one mbarrier and are issued two
+// planes ahead, right after the block barrier that frees their slots (rings
+// of three and four planes measured the same).  H of the plane follows from shared E; its rows and its vectors'
 // last cells go to shared memory (double-buffered by plane, so one barrier
 // per plane suffices), and E follows from those and the previous plane's H
 // kept in registers.
@@ -36,12 +37,24 @@
 // bytes a thread thrash the L1 that the stages leave (256^3 FP32 at 96
 // registers: 0.46 ms a sweep).  For the same reason the profiles and the
 // material table sit in shared memory: a table read that misses L1 stalls
-// every plane for the L2's latency.  z-slab psi rows are stored in vector-aligned slots (SlabExt);
-// cells of a straddling vector outside the slab keep their plain difference.
+// every plane for the L2's latency.  z-slab psi rows are stored in
+// vector-aligned slots (SlabExt); cells of a straddling vector outside the slab keep their plain difference.
 //
 // List cells: the sweep may write any E there (the list kernel overwrites
 // it) but leaves their psi_e alone.  Cells a component's update range leaves
 // out keep their input value.
+//
+// Measured (sweep alone, before = the scalar sweeps): 256^3 FP32 238 us
+// (0.97 GB: 4.1 TB/s) for 265, 128 x 128 x 512 104 for 123; whole steps of
+// 47 x 53 x 61 FP32 13 us for 50, of 64^3 FP64 20 for 54.  What bounds it now
+// (192^3 FP32): DRAM at 4.5 TB/s cold, issue slots 29 % busy with 2.8 warps a
+// scheduler, waits for loads and copies ahead of instruction fetch -- the
+// dependent chain of a plane with few warps to hide it, which registers and
+// stages bound.  Tried: a warp that only issues copies (a plane 1.05 -> 0.87
+// us alone, but its registers cost a resident CTA: 256^3 290 us and more); H
+// and E of the plane before reread from shared memory instead of carried (262
+// for 303 instructions a warp-plane, same time); unrolling by two planes
+// (slower, instruction fetch); 256 threads at 128 registers (290 us).
 //
 // Periodic x wraps the plane index; periodic y reads the wrapped row through
 // one-row boxes behind the tile's.  Every wait is bounded (mbar_wait).

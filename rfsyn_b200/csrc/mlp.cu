@@ -622,6 +622,7 @@ struct fdtd_b200_mlp {
     // training graphs of one step and of GRAPH_STEPS, for batches of graph_b
     cudaGraphExec_t graph = nullptr, graph_n = nullptr;
     int graph_b = 0;
+    unsigned long long graph_l = 0, graph_tc = 0;  // launches a captured step makes, and those on tcgen05
     AdamCfg *cfg = nullptr;
     bool overlap = false;                  // launches are being captured as programmatic dependents
     AdamSeg *segs = nullptr;
@@ -1151,9 +1152,15 @@ static int mlp_capture(fdtd_b200_mlp *m, int B, int steps, cudaGraphExec_t *out)
     cudaGraph_t g = nullptr;
     MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
     m->overlap = !m->tc;
+    const unsigned long long l0 = m->launches, t0 = m->tc_launches;
     int rc = 0;
     for (int s = 0; s < steps && rc == 0; s++) rc = mlp_train_step(m, B, s == 0);
     m->overlap = false;
+    // counted as they are replayed
+    m->graph_l = (m->launches - l0) / steps;
+    m->graph_tc = (m->tc_launches - t0) / steps;
+    m->launches = l0;
+    m->tc_launches = t0;
     const cudaError_t ce = cudaStreamEndCapture(m->st, &g);
     if (rc != 0 || ce != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -1209,7 +1216,10 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
             cudaGraphExec_t *g = many ? &m->graph_n : &m->graph;
             if (!*g && mlp_capture(m, B, many ? GRAPH_STEPS : 1, g) != 0) return -1;
             MCK(cudaGraphLaunch(*g, m->st));
-            s += many ? GRAPH_STEPS : 1;
+            const int n = many ? GRAPH_STEPS : 1;
+            m->launches += n * m->graph_l;
+            m->tc_launches += n * m->graph_tc;
+            s += n;
         }
         done += run;
     }

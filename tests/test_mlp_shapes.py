@@ -81,3 +81,21 @@ def test_training_is_one_sequence():
         assert np.array_equal(used.params(), fresh.params())
         fresh.close()
     used.close()
+
+
+@pytest.mark.parametrize("gemm", ["mma", "tcgen05"])
+def test_launches_of_replayed_steps_count(gemm, monkeypatch):
+    """Every call counts the launches of its steps, also where it replays
+    graphs that an earlier call captured."""
+    monkeypatch.setenv("RFSYN_FDTD_MLP_GEMM", gemm)
+    rng = np.random.default_rng(5)
+    net = rb.Mlp(64, 128, 2, 128, seed=29)
+    net.set_data(rng.uniform(-1, 1, (512, 64)), rng.normal(0, 1, (512, 128)))
+    counts = []
+    for _ in range(3):
+        net.train(9, batch=128, seed=1)
+        counts.append((net.lib.fdtd_b200_mlp_launch_count(net.h), net.tensor_core_launches()))
+    (l0, t0), (l1, t1), (l2, t2) = counts
+    assert l1 - l0 == l2 - l1 > 0 and (l1 - l0) % 9 == 0
+    assert t1 - t0 == t2 - t1 == t0 and (t0 > 0) == (gemm == "tcgen05") and t0 % 9 == 0
+    net.close()

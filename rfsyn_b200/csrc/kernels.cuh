@@ -367,7 +367,9 @@ __host__ __device__ constexpr bool t3_reads(int su, int sv, int sf) {
 // order.  Its 18 curl differences read 36 H samples, 12 a component, 72
 // times: each is loaded once.  The list of the 128 x 128 x 512 unit cell is
 // bound by the latency and the bytes of its gathers (213 MB a step, 3.7 TB/s,
-// cold) rather than by their number: 56.6 -> 55.4 us a step.
+// cold) rather than by their number: 56.6 -> 55.4 us a step.  Fields are
+// plain loads (see overlap.cuh); through the read-only path the step of that
+// cell took the same time (181.6 against 182.1 us).
 template <typename T>
 __device__ __forceinline__ void t3_cell(const Args<T> &a, int cell) {
     const int p[3] = {a.lc_ijk[3 * cell], a.lc_ijk[3 * cell + 1], a.lc_ijk[3 * cell + 2]};
@@ -396,11 +398,11 @@ __device__ __forceinline__ void t3_cell(const Args<T> &a, int cell) {
                 for (int sf = -1; sf <= 1; sf++)
                     if (t3_reads(su, sv, sf))
                         h[f][su + 1][sv + 1][sf + 1] =
-                            __ldg(a.Ho[f] + (c0 + o[(f + 1) % 3][su + 1] + o[(f + 2) % 3][sv + 1] + o[f][sf + 1]));
+                            a.Ho[f][c0 + o[(f + 1) % 3][su + 1] + o[(f + 2) % 3][sv + 1] + o[f][sf + 1]];
     T e[3], r[3][5];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-        e[c] = __ldg(a.E[c] + c0);
+        e[c] = a.E[c][c0];
 #pragma unroll
         for (int q = 0; q < 5; q++) r[c][q] = __ldg(a.t3 + 5 * (long long)tix[c] + q);
     }

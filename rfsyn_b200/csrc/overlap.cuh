@@ -8,6 +8,11 @@
 // kernel's results; grid_wait then holds them until that kernel has ended and
 // its writes are visible.  Every CTA of every step kernel passes grid_wait,
 // also one without work, so the kernels' ends keep their order.
+//
+// A kernel is then resident while the one before it still writes, so nothing
+// that a step writes is read through the read-only path (__ldg, const
+// __restrict__ loads), whose data must not change while the kernel lives and
+// whose loads the compiler may move across grid_wait.
 #pragma once
 #include <cuda_runtime.h>
 

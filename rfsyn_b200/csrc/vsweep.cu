@@ -732,9 +732,12 @@ __device__ __forceinline__ bool v_item(const Args<T> &a, const VShape &sh, const
         }
     }
     if (!__syncthreads_or(failed)) return true;
-    // copies still in flight land (bounded) before the shared memory is released
+    // copies still in flight land (bounded) before the shared memory is
+    // released: the newest V_NH groups at most.  Thread 0's own waits may all
+    // have succeeded (waited 0); the parity of an older group says nothing
+    // once its barrier has moved on, and waiting for it would run out.
     if (tid == 0)
-        for (int g = waited; g < issued; g++) mbar_wait(&bars[g % V_NH], (unsigned)(g / V_NH) & 1u);
+        for (int g = max(waited, issued - V_NH); g < issued; g++) mbar_wait(&bars[g % V_NH], (unsigned)(g / V_NH) & 1u);
     __syncthreads();
     return false;
 }

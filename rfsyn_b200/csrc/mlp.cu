@@ -517,12 +517,13 @@ __global__ void __launch_bounds__(256) k_adam(const AdamSeg *segs, const int2 *b
     const AdamSeg sg = segs[b.x];
     const int i = b.y + 4 * threadIdx.x;
     if (i < sg.n) {
-        const float4 g4 = *reinterpret_cast<const float4 *>(sg.g + i);
-        float4 m4 = *reinterpret_cast<float4 *>(sg.m + i), v4 = *reinterpret_cast<float4 *>(sg.v + i),
-               w4 = *reinterpret_cast<float4 *>(sg.w + i);
-        const float *g = &g4.x;
-        float *m = &m4.x, *v = &v4.x, *w = &w4.x;
-        bf16 h[4];
+        // aligned for the vector accesses also where they are kept in memory
+        alignas(16) float g[4], m[4], v[4], w[4];
+        alignas(8) bf16 h[4];
+        *reinterpret_cast<float4 *>(g) = *reinterpret_cast<const float4 *>(sg.g + i);
+        *reinterpret_cast<float4 *>(m) = *reinterpret_cast<const float4 *>(sg.m + i);
+        *reinterpret_cast<float4 *>(v) = *reinterpret_cast<const float4 *>(sg.v + i);
+        *reinterpret_cast<float4 *>(w) = *reinterpret_cast<const float4 *>(sg.w + i);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             // the contractions nvcc chose for b m + (1 - b) g, written out so
@@ -533,9 +534,9 @@ __global__ void __launch_bounds__(256) k_adam(const AdamSeg *segs, const int2 *b
             w[q] = w[q] - lr * mh / (sqrtf(vh) + a.eps);
             h[q] = __float2bfloat16_rn(w[q]);
         }
-        *reinterpret_cast<float4 *>(sg.m + i) = m4;
-        *reinterpret_cast<float4 *>(sg.v + i) = v4;
-        *reinterpret_cast<float4 *>(sg.w + i) = w4;
+        *reinterpret_cast<float4 *>(sg.m + i) = *reinterpret_cast<const float4 *>(m);
+        *reinterpret_cast<float4 *>(sg.v + i) = *reinterpret_cast<const float4 *>(v);
+        *reinterpret_cast<float4 *>(sg.w + i) = *reinterpret_cast<const float4 *>(w);
         if (sg.w16) *reinterpret_cast<uint2 *>(sg.w16 + i) = *reinterpret_cast<const uint2 *>(h);
         if (sg.w16t) {
             const int r = i / sg.cols, c = i - r * sg.cols;  // four columns of one row (cols a multiple of 4)

@@ -49,7 +49,6 @@ namespace {
 
 constexpr int GK = 64;      // K per stage
 constexpr int GSTAGES = 4;  // stages of the ring
-constexpr int GRAPH_STEPS = 8;  // training steps of the larger graph
 
 enum { EPI_HIDDEN = 0, EPI_OUT = 1, EPI_BWD_GELU = 2, EPI_F32 = 3 };
 
@@ -109,8 +108,8 @@ __device__ __forceinline__ void ldsm4(unsigned (&r)[4], unsigned addr) {
 // give 256 x 512 outputs 128 CTAs (64 x 64 tiles: 32 on 148 SMs), and three
 // 64-deep stages are in flight while one is used: 4.2-7.2 us a product of
 // the 256-row step, cold, against 6.6-17.1 us with 64 x 64 tiles, two 32-deep
-// stages and scalar fragment loads; the whole step 0.21 -> 0.068 ms with the
-// changes around it.  K runs in the same order in every tile, so the tile changes no
+// stages and scalar fragment loads; the whole step 0.19 -> 0.063 ms (calls of
+// 200 steps) with the changes around it.  K runs in the same order in every tile, so the tile changes no
 // result.  Operands in either layout save the transposed copies of weights,
 // activations and gradients.
 template <int EPI, bool TA, bool TB, int BM, int BN>
@@ -620,8 +619,7 @@ struct fdtd_b200_mlp {
     cudaStream_t st = nullptr, st_w = nullptr, st_b = nullptr;  // main; weight and bias gradients
     std::vector<cudaEvent_t> ev_g;         // gradient of layer l ready
     cudaEvent_t ev_w = nullptr, ev_b = nullptr;
-    // training graphs of one step and of GRAPH_STEPS, for batches of graph_b
-    cudaGraphExec_t graph = nullptr, graph_n = nullptr;
+    cudaGraphExec_t graph = nullptr;       // a training step, for batches of graph_b
     int graph_b = 0;
     unsigned long long graph_l = 0, graph_tc = 0;  // launches a captured step makes, and those on tcgen05
     AdamCfg *cfg = nullptr;
@@ -660,17 +658,15 @@ struct Arena {
     }
 };
 
-static void mlp_free_graphs(fdtd_b200_mlp *m) {
-    for (cudaGraphExec_t *g : {&m->graph, &m->graph_n}) {
-        if (*g) cudaGraphExecDestroy(*g);
-        *g = nullptr;
-    }
+static void mlp_free_graph(fdtd_b200_mlp *m) {
+    if (m->graph) cudaGraphExecDestroy(m->graph);
+    m->graph = nullptr;
 }
 
 static void mlp_free_batch(fdtd_b200_mlp *m) {
     cudaFree(m->batch_mem);
     m->batch_mem = nullptr;
-    mlp_free_graphs(m);
+    mlp_free_graph(m);
     m->bmax = 0;
 }
 
@@ -1132,12 +1128,12 @@ extern "C" int fdtd_b200_mlp_set_data(fdtd_b200_mlp_t *m, const float *X, const 
     }
     MCK(cudaMemcpy(m->Y, Y, n * m->n_out * sizeof(float), cudaMemcpyHostToDevice));
     m->n_data = n;
-    mlp_free_graphs(m);
+    mlp_free_graph(m);
     return 0;
 }
 
-static int mlp_train_step(fdtd_b200_mlp *m, int B, bool first) {
-    launch_step(k_gather, dim3(B), dim3(128), 0, m->st, m->overlap && !first, m->X, m->Y, m->perm, (long long)m->n_data,
+static int mlp_train_step(fdtd_b200_mlp *m, int B) {
+    launch_step(k_gather, dim3(B), dim3(128), 0, m->st, false, m->X, m->Y, m->perm, (long long)m->n_data,
                 m->step, B, m->kin, m->n_out, m->act[0], m->actt[0], m->y);
     m->launches++;
     mlp_forward(m, B, true);
@@ -1147,19 +1143,21 @@ static int mlp_train_step(fdtd_b200_mlp *m, int B, bool first) {
     return 0;
 }
 
-// Captures `steps` training steps.  The graphs hold the batch buffers and the
-// data set, not the schedule (cfg, step), so they serve every later call.
-static int mlp_capture(fdtd_b200_mlp *m, int B, int steps, cudaGraphExec_t *out) {
+// Captures a training step.  The graph holds the batch buffers and the data
+// set, not the schedule (cfg, step), so it serves every later call.  A graph
+// of eight steps cost 2 ms more on a network's first call (8 steps of 64 rows:
+// 1.31 against 3.3 ms) and gave nothing back: 200 steps of 256 rows take 12.6
+// against 13.0 ms, of 64 rows 10.7 against 10.4.
+static int mlp_capture(fdtd_b200_mlp *m, int B) {
     cudaGraph_t g = nullptr;
     MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
     m->overlap = !m->tc;
     const unsigned long long l0 = m->launches, t0 = m->tc_launches;
-    int rc = 0;
-    for (int s = 0; s < steps && rc == 0; s++) rc = mlp_train_step(m, B, s == 0);
+    const int rc = mlp_train_step(m, B);
     m->overlap = false;
     // counted as they are replayed
-    m->graph_l = (m->launches - l0) / steps;
-    m->graph_tc = (m->tc_launches - t0) / steps;
+    m->graph_l = m->launches - l0;
+    m->graph_tc = m->tc_launches - t0;
     m->launches = l0;
     m->tc_launches = t0;
     const cudaError_t ce = cudaStreamEndCapture(m->st, &g);
@@ -1168,7 +1166,7 @@ static int mlp_capture(fdtd_b200_mlp *m, int B, int steps, cudaGraphExec_t *out)
         MCK(ce);
         return -1;
     }
-    const cudaError_t e = cudaGraphInstantiate(out, g, 0);
+    const cudaError_t e = cudaGraphInstantiate(&m->graph, g, 0);
     cudaGraphDestroy(g);
     MCK(e);
     return 0;
@@ -1199,7 +1197,7 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
         MCK(cudaMemsetAsync(ly.mb, 0, ly.out * 4, m->st));
         MCK(cudaMemsetAsync(ly.vb, 0, ly.out * 4, m->st));
     }
-    if (m->graph_b != B) mlp_free_graphs(m);
+    if (m->graph_b != B) mlp_free_graph(m);
     m->graph_b = B;
     const size_t per_pass = std::max<size_t>(1, m->n_data / B);
     std::vector<int> perm(m->n_data);
@@ -1212,15 +1210,11 @@ extern "C" int fdtd_b200_mlp_train(fdtd_b200_mlp_t *m, size_t steps, int B, doub
         for (size_t q = m->n_data - 1; q > 0; q--) std::swap(perm[q], perm[splitmix(rs) % (q + 1)]);
         MCK(cudaMemcpyAsync(m->perm, perm.data(), m->n_data * sizeof(int), cudaMemcpyHostToDevice, m->st));
         const size_t run = std::min(per_pass, steps - done);
-        for (size_t s = 0; s < run;) {
-            const bool many = run - s >= (size_t)GRAPH_STEPS;
-            cudaGraphExec_t *g = many ? &m->graph_n : &m->graph;
-            if (!*g && mlp_capture(m, B, many ? GRAPH_STEPS : 1, g) != 0) return -1;
-            MCK(cudaGraphLaunch(*g, m->st));
-            const int n = many ? GRAPH_STEPS : 1;
-            m->launches += n * m->graph_l;
-            m->tc_launches += n * m->graph_tc;
-            s += n;
+        if (!m->graph && mlp_capture(m, B) != 0) return -1;
+        for (size_t s = 0; s < run; s++) {
+            MCK(cudaGraphLaunch(m->graph, m->st));
+            m->launches += m->graph_l;
+            m->tc_launches += m->graph_tc;
         }
         done += run;
     }

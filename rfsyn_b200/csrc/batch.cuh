@@ -268,7 +268,9 @@ static void batch_free_plan(rfb_batch *b) {
 
 // Plan of mode 5, the vector sweep of every scene in one launch: per scene
 // the tile of at most `threads` threads that spends the fewest threads on the
-// grid, and one segment length for the batch: one wave of CTAs where that
+// grid, of those that leave an SM room for V_MB CTAs (one scene's larger tile
+// would halve the CTAs of the whole batch), and one segment length for the
+// batch: one wave of CTAs where that
 // takes at most 16 planes each, else waves of at most 32.  Items of one kind
 // together, the costly kinds first.  96 scenes of 32-96 cells an axis, FP32:
 // 68.5 ms for 96 steps; with 128 threads 68.4-84 (segments of 32-6), with 192
@@ -283,6 +285,7 @@ static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
     maps[1].resize(n);
     double planes = 0;
     int smem = 0;
+    const int args_bytes = b->prec == RFB_FP64 ? v_args_bytes<double>() : v_args_bytes<float>();
     for (size_t s = 0; s < n; s++) {
         rfb_engine *e = b->m[s];
         if (e->g.periodic & 6u) {
@@ -307,6 +310,7 @@ static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
                 if (tr > 1 && nj == (cj + tr - 2) / (tr - 1)) continue;
                 VShape t;
                 if (!v_layout(e, t, nv, tr, cj, ck, threads)) continue;
+                if (v_slots(threads, (int)round_up(t.smem, 16) + args_bytes) < V_MB) continue;
                 const long long tiles = (long long)((nvk + nv - 1) / nv) * nj;
                 const long long cost = tiles * ((tr + 1) * (nv + 1) + threads);
                 if (best < 0 || cost < best) {
@@ -327,7 +331,7 @@ static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
         maps[1][s] = e->vmaps[1];
     }
     smem = (int)round_up(smem, 16);
-    const double slots = 148.0 * v_slots(threads, smem + (b->prec == RFB_FP64 ? v_args_bytes<double>() : v_args_bytes<float>()));
+    const double slots = 148.0 * v_slots(threads, smem + args_bytes);
     if (seg <= 0) {
         const double per_slot = planes / slots;
         seg = std::max(1, (int)ceil(per_slot <= 16 ? per_slot : per_slot / std::max(2.0, ceil(per_slot / 32))));

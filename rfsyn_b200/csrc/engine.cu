@@ -895,6 +895,11 @@ static void launch_tail(rfb_engine *e, int par) {
     p.ts = (T *)e->ts;
     p.n_steps = (long long)e->n_steps;
     p.d_step = e->d_step;
+    if (!e->n_planes && !e->tf_on) {
+        if (e->overlap) launch_step(k_probe_gather<T, true>, dim3(1), dim3(128), 0, e->stream, true, p);
+        else launch_step(k_probe_gather<T, false>, dim3(1), dim3(128), 0, e->stream, false, p);
+        return;
+    }
     const PlaneArgs pl = {e->d_planes, e->n_planes, std::max(1, e->plane_chunks), e->n_probes,
                           (const void *const *)e->d_fout[out], e->d_plane_part, e->d_plane_count};
     const int nb_line = e->tf_on ? (e->tf_m_len + kLineChunk - 1) / kLineChunk : 0;

@@ -354,6 +354,11 @@ __device__ __forceinline__ int slab_in(int q, int lo, int hi, int off, int len, 
     return slab_of(q, lo, hi, off);
 }
 
+__device__ __forceinline__ int slab_in(int q, int lo, int hi, int len, int on) {
+    if (!on || q < 0 || q >= len) return -1;
+    return slab_of(q, lo, hi);
+}
+
 // Per-CTA profile tables in shared memory.
 template <typename T, int TJ>
 struct EdgeShared {
@@ -419,22 +424,22 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
     }
     // slab indices of the own cell (H side: q < n; E side: only swept samples
     // use them, and those have q < n)
-    const int sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+    const int sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.ny, on);
     const int skh = slab_in(k, a.lo_h[2], a.hi_h[2], a.off_h[2], a.nz, on);
-    const int sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.off_m[1], a.ny, on);
+    const int sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.ny, on);
     const int skm = slab_in(k, a.lo_m[2], a.hi_m[2], a.off_m[2], a.nz, on);
     // halo cells: row (j0-1, k) for warp 0, column (j0+tx, k0-1) for warp 1
-    const int sjh_row = slab_in(j0 - 1, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+    const int sjh_row = slab_in(j0 - 1, a.lo_h[1], a.hi_h[1], a.ny, on);
     const int jc = j0 + tx;
-    const int sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+    const int sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.ny, on);
     const int skh_col = slab_in(k0 - 1, a.lo_h[2], a.hi_h[2], a.off_h[2], a.nz, on);
     const int nshy = a.ns_h[1], nshz = a.ns_h[2], nsmy = a.ns_m[1], nsmz = a.ns_m[2];
 
     // psi copies of plane p into stage st
     auto issue_psi = [&](EdgeStage<T, TJ> &st, int p) {
         if (!on || p < 0) return;
-        const int sxh = slab_in(p, a.lo_h[0], a.hi_h[0], a.off_h[0], a.nx, on);
-        const int sxm = slab_in(p, a.lo_m[0], a.hi_m[0], a.off_m[0], a.nx, on);
+        const int sxh = slab_in(p, a.lo_h[0], a.hi_h[0], a.nx, on);
+        const int sxm = slab_in(p, a.lo_m[0], a.hi_m[0], a.nx, on);
         if (own) {
             if (sjh >= 0) {
                 const long long o = ((long long)p * nshy + sjh) * a.pitch + k;
@@ -511,7 +516,7 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
                       const EdgeStage<T, TJ> &cs, const EdgeStage<T, TJ> &ns, bool store) -> T {
         const FusedStage<T, TJ> &cur = cs.f, &nxt = ns.f;
         const T hin = cur.h[c][rr][qq];
-        const int sx = slab_in(i, a.lo_h[0], a.hi_h[0], a.off_h[0], a.nx, on);
+        const int sx = slab_in(i, a.lo_h[0], a.hi_h[0], a.nx, on);
         T dA, dB;
         if (c == 0) {
             if (!(i < a.nx + (px ? 0 : 1) && jj < a.ny && kk < a.nz)) return hin;
@@ -629,7 +634,7 @@ __global__ void __launch_bounds__(32 * TJ, MINB) k_sweep_edge(Args<T> a, FusedDi
             }
             if (!skip) {
                 const T ca = s_tab[code], cb = s_tab[256 + code];
-                const int sxm = slab_in(i, a.lo_m[0], a.hi_m[0], a.off_m[0], a.nx, on);
+                const int sxm = slab_in(i, a.lo_m[0], a.hi_m[0], a.nx, on);
                 if (e_updated(a, 0, i, j, k)) {
                     T tA = xs(sH[2][r][q], sH[2][r - 1][q]);
                     T tB = xs(sH[1][r][q], sH[1][r][q - 1]);

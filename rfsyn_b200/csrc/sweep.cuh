@@ -195,10 +195,10 @@ __device__ __forceinline__ bool q_item(const Args<T> &a, const FusedDims &d, con
         // a body without one axis's slab code serves only tiles whose
         // cells and halos lie outside that slab (the host classifies them)
         if constexpr (YS) {
-            sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
-            sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.off_m[1], a.ny, on);
-            sjh_row = slab_in(jh, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
-            sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.off_h[1], a.ny, on);
+            sjh = slab_in(j, a.lo_h[1], a.hi_h[1], a.ny, on);
+            sjm = slab_in(j, a.lo_m[1], a.hi_m[1], a.ny, on);
+            sjh_row = slab_in(jh, a.lo_h[1], a.hi_h[1], a.ny, on);
+            sjh_col = slab_in(jc, a.lo_h[1], a.hi_h[1], a.ny, on);
             for (int t = tid; t < TR + 1; t += 32 * TJ) {
                 T v[3];
                 prof_at(on ? a.kinv_h[1] : (const T *)nullptr, a.b_h[1], a.a_h[1], j0 - 1 + t, a.ny, v);
@@ -240,7 +240,7 @@ __device__ __forceinline__ bool q_item(const Args<T> &a, const FusedDims &d, con
         int by, bz, bx, sx;
     };
     auto plane_b = [&](int i) -> PlaneB {
-        const int sx = (XS && on) ? slab_in(i, a.lo_h[0], a.hi_h[0], a.off_h[0], a.nx, on) : -1;
+        const int sx = (XS && on) ? slab_in(i, a.lo_h[0], a.hi_h[0], a.nx, on) : -1;
         return PlaneB{i * nshy * pitch, i * (int)ny1 * nshz, sx * plane32, sx};
     };
     T xph[3] = {T(1), T(1), T(0)}, xpm[3] = {T(1), T(1), T(0)};
@@ -377,7 +377,7 @@ __device__ __forceinline__ bool q_item(const Args<T> &a, const FusedDims &d, con
             const unsigned mpl = plane_mask(i);
             const unsigned m = mpl & mjk;
             const PlaneB pb = plane_b(i);
-            const int sxm = (XS && on) ? slab_in(i, a.lo_m[0], a.hi_m[0], a.off_m[0], a.nx, on) : -1;
+            const int sxm = (XS && on) ? slab_in(i, a.lo_m[0], a.hi_m[0], a.nx, on) : -1;
             const int bym = i * nsmy * pitch, bzm = i * (int)ny1 * nsmz, bxm = sxm * plane32;
             // halo cells recomputed this plane: row (j0-1, k) Hx by warp 0,
             // Hz by warp 2; column (j0+tx, k0-1) Hx by warp 1, Hy by warp 3

@@ -632,8 +632,8 @@ struct ProbeArgs {
 // every probe, then advances the device step counter (single block).  LINK:
 // launched as a programmatic dependent.  k_step_tail, which does this and the
 // rest, takes about 3 us longer where its launch does not overlap the kernel
-// before: a step of the fully periodic 46 x 41 x 119 FP64 grid 48.6 us with
-// it, 47.6 with this kernel.
+// before: a step of the fully periodic 46 x 41 x 119 FP64 grid 47.5 us with
+// it, 45.5 with this kernel.
 template <typename T, bool LINK>
 __global__ void __launch_bounds__(128) k_probe_gather(ProbeArgs<T> p) {
     __shared__ int n;

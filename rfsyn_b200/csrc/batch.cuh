@@ -519,12 +519,36 @@ fail:
     return -1;
 }
 
+// A work-queue plan, where every scene is within its sweep's limits.
+static int batch_queue_plan(rfb_batch *b, int tj, int ns, int mode, int seg_int, int seg_edge, int uni) {
+    if (qb_prepare() != 0) {
+        rfb_set_error("cannot configure the batched sweep kernels' shared memory");
+        return -1;
+    }
+    for (size_t s = 0; s < b->m.size(); s++)
+        if (!q_fits(b->m[s])) {
+            rfb_set_error("batch scene %zu too large for the work-queue sweep (32-bit offsets)", s);
+            return -1;
+        }
+    return batch_build_plan(b, tj, ns, mode, seg_int, seg_edge, uni);
+}
+
 // The plan: mode 5 by rule, or the one RFSYN_FDTD_PLAN names -- a work-queue
-// sweep, or "threads,stages,seg_interior,seg_edge,5".  Every plan computes
-// bit-identical fields.
+// sweep, or "threads,stages,seg_interior,seg_edge,5".  A batch with a scene
+// past the vector sweep's limits (v_fits: psi arrays of 2^32 bytes, planes of
+// 2^29) runs on the work-queue sweep, whose limits are wider (q_fits: 2^31
+// elements), by the plan that timing picked for most batches before the vector
+// sweep.  Every plan computes bit-identical fields.
 static int batch_plan(rfb_batch *b) {
     const char *ov = rfb_plan_override();
-    if (!ov) return batch_build_vplan(b, V_BATCH_NT, 0);
+    if (!ov) {
+        // (a periodic y or z axis is refused by either)
+        const bool fits = std::all_of(b->m.begin(), b->m.end(),
+                                      [](const rfb_engine *e) { return (e->g.periodic & 6u) || v_fits(e); });
+        if (fits) return batch_build_vplan(b, V_BATCH_NT, 0);
+        const InteriorVariant v = b->prec == RFB_FP32 ? kQVariantsFp32[0] : kQVariantsFp64[0];
+        return batch_queue_plan(b, v.tj, v.ns, 4, 64, 32, 0);
+    }
     int a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0;
     const int nov = sscanf(ov, "%d,%d,%d,%d,%d,%d", &a1, &a2, &a3, &a4, &a5, &a6);
     if (nov >= 5 && a5 == 5 && a3 > 0 && a1 >= 32 && a1 <= V_NT && a1 % 32 == 0) return batch_build_vplan(b, a1, a3);
@@ -533,7 +557,7 @@ static int batch_plan(rfb_batch *b) {
         rfb_set_error("sweep plan \"%s\" names no work-queue or vector sweep variant", ov);
         return -1;
     }
-    return batch_build_plan(b, a1, a2, a5, a3, a4, a6);
+    return batch_queue_plan(b, a1, a2, a5, a3, a4, a6);
 }
 
 extern "C" void rfb_batch_destroy(rfb_batch_t *b) {
@@ -650,15 +674,6 @@ extern "C" rfb_batch_t *rfb_batch_create(rfb_engine_t **members, size_t n, void 
     CK(cudaMemset(b->d_err, 0, sizeof(int)));
     CK(dmalloc(&b->d_queue, 6 * sizeof(int)));
     CK(cudaMemset(b->d_queue, 0, 6 * sizeof(int)));
-    if (qb_prepare() != 0) {
-        rfb_set_error("cannot configure the batched sweep kernels' shared memory");
-        goto fail;
-    }
-    for (size_t s = 0; s < n; s++)
-        if (!q_fits(members[s])) {
-            rfb_set_error("batch scene %zu too large for the work-queue sweep (32-bit offsets)", s);
-            goto fail;
-        }
     if ((b->prec == RFB_FP64 ? batch_upload_args<double>(b) : batch_upload_args<float>(b)) != 0) goto fail;
     CK(cudaDeviceSynchronize());
     {

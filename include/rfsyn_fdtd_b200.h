@@ -255,7 +255,8 @@ int fdtd_b200_sim_energy(fdtd_b200_sim_t *sim, int x_lo, int x_hi, fdtd_b200_ene
  * precision and step count; the FUSED schedule is used whatever the
  * configuration says; a scene periodic in y or z whose tile halos would wrap
  * is rejected.  The tile plan follows from the scenes' sizes; RFSYN_FDTD_PLAN
- * fixes one: "threads,stages,seg,seg,5", or a work-queue sweep's
+ * fixes one: "threads,stages,seg_interior,seg_edge,5" (32 to 192 threads in
+ * steps of 32, 2 stages), or a work-queue sweep's
  * "rows,ring,seg_interior,seg_edge,mode,single" with mode 2 to 4.  setups / contexts may be NULL, or hold NULL entries. */
 typedef struct fdtd_b200_batch fdtd_b200_batch_t;
 

@@ -271,11 +271,12 @@ static void batch_free_plan(rfb_batch *b) {
 // grid, of those that leave an SM room for V_MB CTAs (one scene's larger tile
 // would halve the CTAs of the whole batch), and one segment length for the
 // batch: one wave of CTAs where that
-// takes at most 16 planes each, else waves of at most 32.  Items of one kind
+// takes at most 16 planes each, else waves of at most 32 (seg and seg_edge,
+// for plain and slab items, where a plan override gives them).  Items of one kind
 // together, the costly kinds first.  96 scenes of 32-96 cells an axis, FP32:
 // 68.5 ms for 96 steps; with 128 threads 68.4-84 (segments of 32-6), with 192
 // and 12-32 planes 72.1-68.8.
-static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
+static int batch_build_vplan(rfb_batch *b, int threads, int seg, int seg_edge) {
     batch_free_plan(b);
     const size_t n = b->m.size();
     std::vector<VShape> shapes(n);
@@ -335,13 +336,14 @@ static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
     if (seg <= 0) {
         const double per_slot = planes / slots;
         seg = std::max(1, (int)ceil(per_slot <= 16 ? per_slot : per_slot / std::max(2.0, ceil(per_slot / 32))));
+        seg_edge = seg;
     }
     b->n_vplain = 0;
     for (size_t s = 0; s < n; s++) {
         int cj, ck, ci;
         v_extents(b->m[s], b->m[s]->active, &cj, &ck, &ci);
-        const int sg = std::min(seg, v_max_seg(b->m[s]));
-        v_items(b->m[s], shapes[s], ci, sg, sg, (int)s, items, &b->n_vplain);
+        const int most = v_max_seg(b->m[s]);
+        v_items(b->m[s], shapes[s], ci, std::min(seg, most), std::min(seg_edge, most), (int)s, items, &b->n_vplain);
     }
     auto rank = [](const VItem &x) { return x.kind & V_X ? 0 : 4 - x.kind; };
     std::stable_sort(items.begin(), items.end(), [&](const VItem &x, const VItem &y) {
@@ -352,7 +354,8 @@ static int batch_build_vplan(rfb_batch *b, int threads, int seg) {
     b->uni = 1;
     b->tj = threads;
     b->ns = V_NH;
-    b->seg_int = b->seg_edge = seg;
+    b->seg_int = seg;
+    b->seg_edge = seg_edge;
     b->v_nt = threads;
     b->v_smem = smem;
     b->n_vitems = (int)items.size();
@@ -545,13 +548,14 @@ static int batch_plan(rfb_batch *b) {
         // (a periodic y or z axis is refused by either)
         const bool fits = std::all_of(b->m.begin(), b->m.end(),
                                       [](const rfb_engine *e) { return (e->g.periodic & 6u) || v_fits(e); });
-        if (fits) return batch_build_vplan(b, V_BATCH_NT, 0);
+        if (fits) return batch_build_vplan(b, V_BATCH_NT, 0, 0);
         const InteriorVariant v = b->prec == RFB_FP32 ? kQVariantsFp32[0] : kQVariantsFp64[0];
         return batch_queue_plan(b, v.tj, v.ns, 4, 64, 32, 0);
     }
     int a1 = 0, a2 = 0, a3 = 0, a4 = 0, a5 = 0, a6 = 0;
     const int nov = sscanf(ov, "%d,%d,%d,%d,%d,%d", &a1, &a2, &a3, &a4, &a5, &a6);
-    if (nov >= 5 && a5 == 5 && a3 > 0 && a1 >= 32 && a1 <= V_NT && a1 % 32 == 0) return batch_build_vplan(b, a1, a3);
+    if (nov >= 5 && a5 == 5 && a2 == V_NH && a3 > 0 && a4 > 0 && a6 >= 0 && a6 <= 1 && a1 >= 32 && a1 <= V_NT && a1 % 32 == 0)
+        return batch_build_vplan(b, a1, a3, a4);
     if (nov < 5 || a5 < 2 || a5 > 4 || a3 <= 0 || a4 <= 0 || a6 < 0 || a6 > 1 ||
         !plan_variant_known(b->prec, a1, a2, a5)) {
         rfb_set_error("sweep plan \"%s\" names no work-queue or vector sweep variant", ov);

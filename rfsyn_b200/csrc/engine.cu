@@ -1519,6 +1519,10 @@ fail:
 static int build_sweep_plan(rfb_engine *e, int active, int tj, int ns, int tma, int seg_int, int seg_edge,
                             int uni = 0, int i2 = 0) {
     if (tma == 5) {
+        if (i2) {
+            rfb_set_error("the two-rows interior sweep needs an FP32 plan of mode 2 or 3");
+            return -1;
+        }
         const VPick v = {tj, ns, seg_int, seg_edge};
         return v_build_plan(e, active, &v);
     }

@@ -779,7 +779,8 @@ def run_profile(args) -> None:
         setups = [scenes.scene_setup(x) for x in ws]
         b = rb.Batch([scenes.run_config(x) for x in ws], [st.ptr if st else None for st in setups])
         bi = b.info()
-        print(f"batch plan: rows {bi.tile_j}, ring {bi.ring_depth}, scenes {bi.scenes}, cells {bi.cells}", flush=True)
+        print(f"batch plan: {bi.tile_j},{bi.ring_depth},{bi.seg_interior},{bi.seg_edge},{bi.mode},{bi.unified} "
+              f"(mode 5: threads, stages), scenes {bi.scenes}, cells {bi.cells}", flush=True)
         sweep_ms, other_ms = b.time_kernels(steps)
         b.close()
         print(f"c4 x{args.scenes}: {steps} steps, sweep {sweep_ms / steps:.3f} ms/step, other {other_ms / steps:.3f} ms/step")

@@ -209,7 +209,12 @@ static inline int qb_prepare() {
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr int V_BATCH_NT = 192;  // threads of the vector sweep's CTAs
+// Threads of the vector sweep's CTAs.  us a step at 192 / best of 160 / best of
+// 128 threads (segments 12-32): 96 scenes of 32-96 cells an axis FP32 602 /
+// 660 / 623, FP64 1113 / 1167 / 1339; 12 of 60-96 FP32 140 / 151 / 140, FP64
+// 226 / 250 / 278; 30 of 40-80 FP32 184 / 202 / 190, FP64 310 / 334 / 377.
+// Batches of few small scenes can want fewer: 20 of 32-60 FP32 75 / 79 / 67.
+constexpr int V_BATCH_NT = 192;
 
 struct rfb_batch {
     std::vector<rfb_engine *> m;  // members (owned)

@@ -1294,8 +1294,8 @@ static int v_max_seg(const rfb_engine *e) {
 
 // Tile shape and segment length, by the planes W that a CTA slot gets.
 //
-// Large grids (W > V_DENSE): CTAs of at most 128 threads, three to an SM, that
-// leave each other's barriers alone, on tiles 8 vectors wide where the grid
+// Large grids (W > V_DENSE): CTAs of at most 128 threads, three to an SM (two
+// in FP64 with material tables), that leave each other's barriers alone, on tiles 8 vectors wide where the grid
 // allows: their rows are whole 128-byte lines, so no two CTAs write parts of
 // one.  Of such shapes (13 x 8 on most grids) the one with the fewest tiles,
 // others counting 1.1 (measured 1.02-1.1).  Segments of three quarters of W,
@@ -1303,15 +1303,23 @@ static int v_max_seg(const rfb_engine *e) {
 // longer ones leave slots empty at the end.  Sweep alone, against the small
 // grids' rule: 256^3 FP32 238 for 245 us, a 128 x 128 x 512 unit cell 104 for
 // 118, 150 x 131 x 170 FP64 112 for 124, 150^3 FP32 64 for 80, 128^3 49 for
-// 56, 112^3 40 for 50, 96^3 FP64 44 for 52, 90^3 FP64 (W = 8.2) 40 for 42.
+// 56, 112^3 40 for 50, 96^3 FP64 44 for 52, 90^3 FP64 (W = 8.2) 40 for 42.  The
+// other way: 200^3 FP64 226 for 215 (a step 229 us, with the scalar sweeps 259).
+// 200^3 FP32 lands on 20 x 5 tiles by 2 % of the count and gains nothing on the
+// scalar sweeps (174 us a step both), against 0.8 of their time on 192^3 and
+// 224^3.
 //
 // Small grids: a CTA takes about the same time a plane however small its tile
 // (the plane's chain of dependent instructions, 1.1-1.4 us), so the rule
 // minimises the planes the busiest slot marches, one more than its length per
 // item, weighted with the halo threads of the shape: 96^3 FP32 (W = 5) 29.9 us
 // for 31.6 on 13 x 8, 200 x 200 x 30 (W = 7.2) the same on both.  Where y is
-// periodic, no slab planes contend and the line lies higher: 77 x 91 x 203
-// (W = 8.5) 26.8 for 28.0, 96 x 96 x 203 (W = 12) 35.0 for 34.7 the other way.
+// periodic W separates the two poorly.  Of 18 such grids with W from 7.6 to 18,
+// the line at 10 puts 11 on their better side; the others lose 4-18 % on it:
+// 77 x 91 x 203 (W = 8.5) takes 25.7 us a step for 24.0 on 13 x 8, 80 x 110 x
+// 180 (W = 13) 30.0 for 25.4 on 11 x 15.  At 8 it would put 11 there as well
+// (60 x 100 x 130 FP64, W = 8.8, 29.8 for 28.6; 150 x 60 x 180, W = 9.1, 31.2
+// for 27.2).
 constexpr double V_DENSE = 8.0, V_DENSE_PY = 10.0;
 constexpr int V_REGS = 168;  // registers a thread of k_vsweep holds at most
 
@@ -1649,6 +1657,7 @@ static int autotune(rfb_engine *e, int active) {
         int tma;
     };
     std::vector<Cand> vars;
+    // mode 4 here: grids past v_fits alone
     const bool qok = q_fits(e), narrow = qok && !(e->g.periodic & 6u);
     if (e->prec == RFB_FP32) {
         if (qok)

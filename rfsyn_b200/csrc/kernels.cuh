@@ -372,10 +372,10 @@ __host__ __device__ constexpr bool t3_reads(int su, int sv, int sf) {
 // The three components of a cell whose samples are all 3x3 samples (no
 // source, no TF/SF term): e_tensor3 for c = 0, 1, 2 with the same operation
 // order.  Its 18 curl differences read 36 H samples, 12 a component, 72
-// times: each is loaded once.  The list of the 128 x 128 x 512 unit cell is
-// bound by the latency and the bytes of its gathers (213 MB a step, 3.7 TB/s,
-// cold) rather than by their number: 56.6 -> 55.4 us a step.  Fields are
-// plain loads (see overlap.cuh); through the read-only path the step of that
+// times: each is loaded once.  The list of a 128 x 128 x 512 unit cell (1.03 M
+// cells) is bound by the latency and the bytes of its gathers (213 MB a step,
+// 3.7 TB/s, cold) rather than by their number: 56.6 -> 55.4 us a step.  Fields
+// are plain loads (see overlap.cuh); through the read-only path the step of that
 // cell took the same time (181.6 against 182.1 us).
 template <typename T>
 __device__ __forceinline__ void t3_cell(const Args<T> &a, int cell) {

@@ -6,8 +6,10 @@
 // kernel's CTAs start once every CTA of the kernel before it has started
 // (grid_launch_next, first thing in each kernel) and do what reads no other
 // kernel's results; grid_wait then holds them until that kernel has ended and
-// its writes are visible.  Every CTA of every step kernel passes grid_wait,
-// also one without work, so the kernels' ends keep their order.
+// its writes are visible.  Every CTA of a kernel that is launched with the link
+// passes grid_wait, also one without work, so the kernels' ends keep their
+// order.  Kernels launched without it (the network's bias sums and weight
+// gradients on streams of their own, its update) stand behind full edges.
 //
 // A kernel is then resident while the one before it still writes, so nothing
 // that a step writes is read through the read-only path (__ldg, const

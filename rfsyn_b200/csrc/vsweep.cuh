@@ -1,5 +1,5 @@
-// vsweep.cuh -- H+E sweep of vector cells: the sweep every grid without a
-// periodic z axis runs on (sweep mode 5).
+// vsweep.cuh -- H+E sweep of vector cells (sweep mode 5): what grids without a
+// periodic z axis run on, up to its 32-bit limits (v_fits).
 //
 // One launch per time step takes the whole grid.  A CTA marches one item --
 // a tile of TR rows x NV vectors in (j, k), a range of planes -- along i; a
@@ -46,11 +46,14 @@
 //
 // Measured (sweep alone, before = the scalar sweeps): 256^3 FP32 238 us
 // (0.97 GB: 4.1 TB/s) for 265, 128 x 128 x 512 104 for 123; whole steps of
-// 47 x 53 x 61 FP32 13 us for 50, of 64^3 FP64 20 for 54.  What bounds it now
-// (192^3 FP32): DRAM at 4.5 TB/s cold, issue slots 29 % busy with 2.8 warps a
-// scheduler, waits for loads and copies ahead of instruction fetch -- the
-// dependent chain of a plane with few warps to hide it, which registers and
-// stages bound.  Tried: a warp that only issues copies (a plane 1.05 -> 0.87
+// 47 x 53 x 61 FP32 13 us for 50, of 64^3 FP64 20 for 54.  What bounds it now:
+// on 256^3 FP32 it moves 714 MB in and 441 MB out in 227 us cold, 5.1 TB/s or
+// 0.79 of the copy rate, where one pass would read 494 MB -- the rest are halo
+// lines fetched again (a box is (TR + 2)(NV + 2) vectors and starts one vector
+// before a line).  On 192^3 FP32 DRAM runs at 4.5 TB/s cold, issue slots are 29 %
+// busy with 2.8 warps a scheduler, waits for loads and copies ahead of
+// instruction fetch: the dependent chain of a plane with few warps to hide it,
+// which registers and stages bound.  Tried: a warp that only issues copies (a plane 1.05 -> 0.87
 // us alone, but its registers cost a resident CTA: 256^3 290 us and more); H
 // and E of the plane before reread from shared memory instead of carried (262
 // for 303 instructions a warp-plane, same time); unrolling by two planes

@@ -1146,8 +1146,9 @@ static int mlp_train_step(fdtd_b200_mlp *m, int B) {
 // Captures a training step.  The graph holds the batch buffers and the data
 // set, not the schedule (cfg, step), so it serves every later call.  A graph
 // of eight steps cost 2 ms more on a network's first call (8 steps of 64 rows:
-// 1.31 against 3.3 ms) and gave nothing back: 200 steps of 256 rows take 12.6
-// against 13.0 ms, of 64 rows 10.7 against 10.4.
+// 1.31 against 3.3 ms) and gave little back: 200 steps of 256 rows take 12.6
+// against 13.0 ms, of 64 rows 10.7 against 10.4, 43 steps of 64 rows on two
+// layers of 128 1.30 against 1.23.
 static int mlp_capture(fdtd_b200_mlp *m, int B) {
     cudaGraph_t g = nullptr;
     MCK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
